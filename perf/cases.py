@@ -4,8 +4,8 @@ A case is a dict of plain values.  ``path`` says which call it is:
 
 * ``march``     ``B200Backend.run``: a chunk of steps of one solve, host state in and out, as
                 ``march.solve`` (and the host solver this backend plugs into) calls it;
-* ``batch``     ``BatchSolver``: a design sweep's members marched together for ``steps`` steps, then
-                every member's observables;
+* ``batch``     ``BatchSolver``: a design sweep's members marched together for ``steps`` steps (the
+                observables, taken once after tens of thousands of steps, are left out);
 * ``stage``     ``BatchSolver`` with one member: a device-resident step of one large mesh of random
                 admissible states, about half of whose elements the limiter works on;
 * ``residual``  ``AdjointModel.residual``: one residual of a device-resident state;
@@ -258,10 +258,8 @@ def run(s):
         s.solver.reset()
         s.solver.run()
         res = s.solver.results(with_state=False)
-        obs = s.solver.observables()
         return {"states": [S[0] for _, S in s.solver.buffers],  # every member's state, bucket by bucket
-                "residuals": np.array([r.residual for r in res]), "iterations": np.array([r.iterations for r in res]),
-                "observables": np.array([[o[k] for k in OBSERVABLES] for o in obs])}
+                "residuals": np.array([r.residual for r in res]), "iterations": np.array([r.iterations for r in res])}
     if s.path == "stage":
         s.solver.reset()
         s.solver.run()
@@ -277,9 +275,6 @@ def run(s):
     n = s.case["steps"]
     lam, rel, its, _ = s.march.solve(tolerance=1e-8, max_iterations=n, check_interval=n)
     return {"lam": lam, "rel": rel, "iterations": its}
-
-
-OBSERVABLES = ("thrust", "mass_flow_in", "mass_flow_out", "exit_mach", "exit_pressure_ratio", "entropy_error")
 
 
 # ------------------------------------------------------------------ what a pass cannot do without
