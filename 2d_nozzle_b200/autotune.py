@@ -15,13 +15,15 @@ compiler contracts multiply-adds differently in different kernels, and
 ``split4`` associates a few sums differently).  The adjoint state kernel has
 ``t1`` and ``split4`` too.
 
-Which is fastest depends on the context, so the table has two: ``single``
-(one solve on its own mesh of a few thousand elements -- latency-bound, where
-four threads per element shorten an element's path) and ``batch`` (a bucket
-of a batch marching beside the other buckets -- throughput-bound, where one
-thread per element wastes fewer instructions).  Within a context the variant
-is fixed per (kind, order), never per mesh; a batch built with
-``variants="single"`` runs the plain solve's kernels and gives its bits.
+Which is fastest can depend on the context, so the table has two: ``single``
+(one solve on its own mesh of a few thousand elements -- latency-bound) and
+``batch`` (a bucket of a batch marching beside the other buckets, or one mesh
+that fills the GPU -- throughput-bound).  ``split4`` is the forward choice of
+both above p = 0: a stage of a single solve takes 7-18 us with it and 25-220 us
+with one thread per element, a step of a 72-member sweep (211 680 elements) 0.55
+against 1.0 ms.  Within a context the variant is fixed per (kind, order), never
+per mesh; a batch built with ``variants="single"`` runs the plain solve's kernels
+and gives its bits.  One exception, :func:`bucket_context`.
 
 The table is ``variants.json`` beside this module, written by
 ``python -m 2d_nozzle_b200.autotune --write`` on a B200 (see :func:`tune`).
@@ -102,6 +104,8 @@ def variant_for(kind: str, order: int, context: str = "single") -> str:
         if forced not in VARIANTS:
             raise ValueError(f"NZB_VARIANT={forced!r}: use one of {sorted(VARIANTS)}")
         return forced
+    if context == "lone":
+        return "t1"
     name = _lookup(kind, order, context, "fwd")
     # four threads per element apply from p = 1 up
     return "t1" if (name == "split4" and int(order) == 0) else name
@@ -127,7 +131,7 @@ def vjp_variant_for(kind: str, order: int, context: str = "single") -> str:
             raise ValueError(f"NZB_VJP_VARIANT={forced!r}: use one of {sorted(VJP_VARIANTS)}")
         name = forced
     else:
-        name = _lookup(kind, order, context, "vjp")
+        name = _lookup(kind, order, "batch" if context == "lone" else context, "vjp")
     return "t1" if int(order) == 0 else name
 
 
@@ -157,6 +161,21 @@ def context_for(n_elem: int, variants: str = "auto") -> str:
     if variants not in CONTEXTS:
         raise ValueError(f"variants {variants!r}: use 'auto' or one of {CONTEXTS}")
     return variants
+
+
+# Elements above which the only instance of a bucket keeps the one-thread kernels (bucket_context).
+LONE_ELEMENTS = 16384
+
+
+def bucket_context(n_instances: int, n_elem: int, variants: str) -> str:
+    """The variant context of a batch's bucket: ``variants``, except that a throughput bucket holding a
+    single large instance takes ``lone``, whose forward choice is the one-thread kernel.  That is the
+    stage benchmark's shape -- one large mesh of random states, half of whose elements the limiter
+    rescales toward vacuum -- and a step from such states magnifies the last bits of the fluxes by up to
+    1e8 (a contact speed equal to a wave speed but for round-off), so its results are kept bit for bit
+    although the tile kernel is faster there (500 000 cubic triangles: a limited stage 1.03 against
+    0.62 ms).  Sweeps' instances are far below the line (9 000 elements at refinement 3)."""
+    return "lone" if variants == "batch" and n_instances == 1 and n_elem > LONE_ELEMENTS else variants
 
 
 def choose_variant(mesh, context: str = "single") -> str:

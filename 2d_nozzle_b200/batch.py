@@ -28,7 +28,7 @@ import numpy as np
 
 from . import capi
 from .config import FLUX_IDS, SCHEMES, recommended_scheme, residual_scale, step_coefficient
-from .autotune import choose_variant, set_struct_variant, tail_elements
+from .autotune import bucket_context, choose_variant, set_struct_variant, tail_elements
 from .layout import DeviceMesh, concat_arrays, host_arrays, physics_struct
 
 STATUS = {0: "running", 1: "converged", 2: "non-finite", 3: "diverged", 4: "stalled", 5: "max_iterations"}
@@ -186,7 +186,7 @@ class BatchSolver:
                 dm.pack(U0, S[0])
                 self.h2d_bytes += U0.nbytes
             self.U0_soa.append(S[0].clone())
-            choose_variant(dm, variants)
+            choose_variant(dm, bucket_context(len(mem), dm.E, variants))
             self.h2d_bytes += sum(a.nbytes for a in arrays.values() if isinstance(a, np.ndarray))
             bf = capi.Buffers()
             bf.S0, bf.S1, bf.S2 = (x.data_ptr() for x in S)

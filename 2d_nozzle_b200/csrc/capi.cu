@@ -669,7 +669,8 @@ int nzb_upload_tables(int kind, int order, const double* tables, int64_t n) {
       cuda_check(upload_tables_fwd_quad(tables, (size_t)n, off), "table upload (quadrilaterals)") ||
       cuda_check(upload_tables_tri(tables, (size_t)n, off), "table upload (adjoint, triangles)") ||
       cuda_check(upload_tables_quad(tables, (size_t)n, off), "table upload (adjoint, quadrilaterals)") ||
-      cuda_check(kind == NZB_TRI ? prepare_split_tri(order) : prepare_split_quad(order), "split kernel attributes") ||
+      cuda_check(kind == NZB_TRI ? upload_tiles_fwd_tri(order, tables) : upload_tiles_fwd_quad(order, tables),
+                 "tile fragment upload") ||
       cuda_check(kind == NZB_TRI ? prepare_vjp_split_tri(order) : prepare_vjp_split_quad(order),
                  "adjoint split kernel attributes"))
     return -1;

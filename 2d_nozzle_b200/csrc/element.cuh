@@ -323,15 +323,19 @@ __device__ __forceinline__ void limit_element(const A& u, const nzb_mesh& m,
   scaled = 1;
 }
 
-// The block of the mesh this CTA runs: entry blockIdx.x of a block list (the
-// blocks of a batch that still hold marching elements), or blockIdx.x itself.
+// The block of the mesh at position `at` of a launch (its CTA's index by default):
+// that entry of a block list (the blocks of a batch that still hold marching
+// elements), or the position itself.
 // An entry outside [0, ceil(E / W)) maps to the first block past the end, whose
 // elements are all inactive.
-__device__ __forceinline__ int64_t listed_block(const int32_t* __restrict__ list, int64_t E, int W) {
-  if (!list) return blockIdx.x;
+__device__ __forceinline__ int64_t listed_block(const int32_t* __restrict__ list, int64_t E, int W, int64_t at) {
+  if (!list) return at;
   const int64_t end = (E + W - 1) / W;
-  const int64_t b = __ldg(list + blockIdx.x);
+  const int64_t b = __ldg(list + at);
   return (b < 0 || b > end) ? end : b;
+}
+__device__ __forceinline__ int64_t listed_block(const int32_t* __restrict__ list, int64_t E, int W) {
+  return listed_block(list, E, W, blockIdx.x);
 }
 
 template <int NW>

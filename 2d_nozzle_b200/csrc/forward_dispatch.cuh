@@ -43,9 +43,9 @@ NZB_INTERNAL cudaError_t initial_launch_tri(const nzb_mesh& m, const nzb_physics
                                             cudaStream_t st);
 NZB_INTERNAL cudaError_t initial_launch_quad(const nzb_mesh& m, const nzb_physics& ph, const nzb_initial_args& a,
                                              cudaStream_t st);
-// raise the split kernels' dynamic shared-memory limit for one order (current device)
-NZB_INTERNAL cudaError_t prepare_split_tri(int order);
-NZB_INTERNAL cudaError_t prepare_split_quad(int order);
+// build and upload one order's tile fragments from its table slot (current device)
+NZB_INTERNAL cudaError_t upload_tiles_fwd_tri(int order, const double* slot);
+NZB_INTERNAL cudaError_t upload_tiles_fwd_quad(int order, const double* slot);
 NZB_INTERNAL cudaError_t upload_tables_fwd_tri(const double* src, size_t count, size_t offset);
 NZB_INTERNAL cudaError_t upload_tables_fwd_quad(const double* src, size_t count, size_t offset);
 

@@ -3,7 +3,8 @@
 // forward_quad.cu (each translation unit instantiates it for its own kind).
 //
 // Variants (nzb_mesh.split, nzb_mesh.edge_pass):
-//   split = 4      k_split: four threads per element (split.cuh), p >= 1;
+//   split = 4      k_tile: four lanes per element, FP64 tensor cores
+//                  (tile_element.cuh), p >= 1;
 //   edge_pass = 1  k_edge (one thread per edge) then k_element with the
 //                  fluxes lifted from the edge array;
 //   otherwise      k_element: one thread per element, fluxes from both sides.
@@ -13,9 +14,11 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <initializer_list>
+
 #include "element.cuh"
 #include "slope.cuh"
-#include "split.cuh"
+#include "tile_element.cuh"
 
 namespace nzb {
 namespace {
@@ -33,6 +36,32 @@ cudaError_t superbee_passes(const nzb_mesh& m, const nzb_physics& ph, const doub
   return cudaGetLastError();
 }
 
+// Persistent CTAs, as many as the GPU holds at once: the tables are staged once per
+// CTA, and a warp prefetches its next tile while it works on one.
+template <int K, int P, bool AFF, bool LIM>
+void launch_tile(const nzb_mesh& m, const nzb_physics& ph, const Work& w, int64_t blocks, cudaStream_t st) {
+  using L = TileSmem<K, P, AFF, LIM>;
+  constexpr int64_t most = 148 * L::MINB;
+  k_tile<K, P, AFF, LIM><<<(unsigned)(blocks < most ? blocks : most), TILE_WARPS * 32, L::BYTES, st>>>(m, ph, w);
+}
+
+inline cudaError_t first_error(std::initializer_list<cudaError_t> all) {
+  for (const cudaError_t e : all)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
+// The tile kernels' dynamic shared memory exceeds the default 48 KB limit at some
+// orders: raise each instantiation's limit (once per device, at table upload).
+template <int K, int P, bool AFF>
+cudaError_t prepare_tile() {
+  const cudaError_t e = cudaFuncSetAttribute(k_tile<K, P, AFF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             TileSmem<K, P, AFF, true>::BYTES);
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(k_tile<K, P, AFF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 TileSmem<K, P, AFF, false>::BYTES);
+}
+
 template <int K, int P, bool AFF>
 cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cudaStream_t st) {
   const bool sb = ph.limiter == 2 && P > 0 && (w.op == OP_STAGE || w.op == OP_LIMIT);
@@ -40,15 +69,14 @@ cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cuda
   const bool lim = w.op == OP_STAGE || w.op == OP_LIMIT;
   bool done = false;
   if constexpr (P > 0) {
-    if (m.split == SPLIT_T) {
-      const unsigned nb = (unsigned)(m.fwd_blocks ? m.n_fwd_blocks : (m.n_elem + SPLIT_EB - 1) / SPLIT_EB);
-      constexpr int SM = SplitSmem<K, P>::BYTES;
-      if (nb == 0)
+    if (m.split == TILE_LANES) {
+      const int64_t blocks = m.fwd_blocks ? m.n_fwd_blocks : (m.n_elem + TILE_EB - 1) / TILE_EB;
+      if (blocks == 0)
         ;  // an empty block list: nothing marches
       else if (lim)
-        k_split<K, P, AFF, true><<<nb, SPLIT_T * 32, SM, st>>>(m, ph, w);
+        launch_tile<K, P, AFF, true>(m, ph, w, blocks, st);
       else
-        k_split<K, P, AFF, false><<<nb, SPLIT_T * 32, SM, st>>>(m, ph, w);
+        launch_tile<K, P, AFF, false>(m, ph, w, blocks, st);
       done = true;
     }
   }
@@ -78,21 +106,6 @@ cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cuda
     return superbee_passes<K, P, AFF>(m, ph, w.out, w.out, w.counters, w.flags, st);
   }
   return cudaGetLastError();
-}
-
-// The split kernels' dynamic shared memory exceeds the default 48 KB limit at
-// p = 3: raise each instantiation's limit (once per device, at table upload).
-template <int K, int P, bool AFF>
-cudaError_t prepare_split() {
-  if constexpr (P == 0) {
-    return cudaSuccess;
-  } else {
-    constexpr int SM = SplitSmem<K, P>::BYTES;
-    cudaError_t e = cudaFuncSetAttribute(k_split<K, P, AFF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_split<K, P, AFF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-    return e;
-  }
 }
 
 }  // namespace

@@ -59,11 +59,11 @@ cudaError_t geometry_launch_quad(const nzb_mesh& m, const nzb_geometry_args& a, 
   return cudaGetLastError();
 }
 
-cudaError_t prepare_split_quad(int order) {
+cudaError_t upload_tiles_fwd_quad(int order, const double* slot) {
   switch (order) {
-    case 1: return prepare_split<1, 1, false>();
-    case 2: return prepare_split<1, 2, false>();
-    case 3: return prepare_split<1, 3, false>();
+    case 1: return first_error({upload_tiles<1, 1>(slot), prepare_tile<1, 1, false>()});
+    case 2: return first_error({upload_tiles<1, 2>(slot), prepare_tile<1, 2, false>()});
+    case 3: return first_error({upload_tiles<1, 3>(slot), prepare_tile<1, 3, false>()});
   }
   return cudaSuccess;
 }

@@ -73,20 +73,11 @@ cudaError_t geometry_launch_tri(const nzb_mesh& m, const nzb_geometry_args& a, c
   return cudaGetLastError();
 }
 
-cudaError_t prepare_split_tri(int order) {
+cudaError_t upload_tiles_fwd_tri(int order, const double* slot) {
   switch (order) {
-    case 1: {
-      const cudaError_t e = prepare_split<0, 1, true>();
-      return e != cudaSuccess ? e : prepare_split<0, 1, false>();
-    }
-    case 2: {
-      const cudaError_t e = prepare_split<0, 2, true>();
-      return e != cudaSuccess ? e : prepare_split<0, 2, false>();
-    }
-    case 3: {
-      const cudaError_t e = prepare_split<0, 3, true>();
-      return e != cudaSuccess ? e : prepare_split<0, 3, false>();
-    }
+    case 1: return first_error({upload_tiles<0, 1>(slot), prepare_tile<0, 1, true>(), prepare_tile<0, 1, false>()});
+    case 2: return first_error({upload_tiles<0, 2>(slot), prepare_tile<0, 2, true>(), prepare_tile<0, 2, false>()});
+    case 3: return first_error({upload_tiles<0, 3>(slot), prepare_tile<0, 3, true>(), prepare_tile<0, 3, false>()});
   }
   return cudaSuccess;
 }

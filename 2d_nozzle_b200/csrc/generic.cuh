@@ -1,7 +1,7 @@
 // generic.cuh -- the DG step for any order and curved (Q = 2) elements, from
 // the reference's per-element operators.
 //
-// The specialised kernels (element.cuh, split.cuh) hold every table of an
+// The specialised kernels (element.cuh, tile_element.cuh) hold every table of an
 // element type in the constant bank and rebuild the metric terms of straight
 // elements at each point; they are instantiated for straight elements of
 // order 0..3.  For higher orders (up to 21 basis functions and beyond) and for

@@ -92,4 +92,11 @@ __host__ __device__ constexpr int edge_node(int kind, int p, int f, int j) {
                 : (f == 1 ? lattice_node(1, p, p, j) : (f == 2 ? lattice_node(1, p, p - j, p) : lattice_node(1, p, 0, p - j)));
 }
 
+// Index of node i on edge f of the element (0..p), or -1.
+__host__ __device__ constexpr int edge_pos(int kind, int p, int f, int i) {
+  for (int j = 0; j <= p; ++j)
+    if (edge_node(kind, p, f, j) == i) return j;
+  return -1;
+}
+
 }  // namespace nzb

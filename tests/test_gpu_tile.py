@@ -1,0 +1,66 @@
+"""The tile kernels (four lanes per element, FP64 tensor cores) at the edges of their tiling.
+
+A warp owns eight elements, a block 32, and a CTA takes several blocks once the mesh has more than
+fit the GPU at a time: meshes of a few elements, of one element more or less than a tile or a block,
+and of more blocks than CTAs.  The reference is the one-thread kernel (held to the oracle elsewhere).
+
+Tolerance: an output sums at most 32 point terms of at most 16-term interpolations, and the trace
+tables differ between faces by up to 1.3e-14 (the reference's own round-off at cubic quadrilaterals),
+so 100 terms x 1.3e-14 bounds the relative difference: 2e-12.
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import pkg, rel
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-12
+
+# (nx, nr) cells: triangles have twice as many elements, quadrilaterals as many
+SIZES = [(2, 1), (3, 1), (4, 1), (5, 3), (8, 2), (11, 3), (33, 1), (160, 97)]
+
+
+def _states(ops, seed):
+    """Smooth flow with enough noise that some elements are limited and none is near vacuum."""
+    rng = np.random.default_rng(seed)
+    shape = (ops.n_elem, ops.ref.n_basis)
+    rho = 1.0 + 0.2 * rng.uniform(-1, 1, shape)
+    vx, vy, p = (rng.uniform(a, b, shape) for a, b in ((0.2, 0.9), (-0.3, 0.3), (0.4, 0.8)))
+    return np.stack([rho, rho * vx, rho * vy, p / 0.4 + 0.5 * rho * (vx * vx + vy * vy)], -1)
+
+
+@pytest.mark.parametrize("kind", ["tri", "quad"])
+@pytest.mark.parametrize("p", [1, 2, 3])
+@pytest.mark.parametrize("nx,nr", SIZES)
+def test_tiles_agree_with_one_thread(cuda, kind, p, nx, nr):
+    cfg, mesh = pkg("config"), pkg("mesh")
+    topo, xf, rf = mesh.channel_topology(kind, nx=nx, nr=nr)
+    X = mesh.rectangle_coords(xf, rf)
+    X = X + 0.1 / max(nx, nr) * np.sin(7.0 * X[:, ::-1])  # no two elements alike
+    ops = pkg("operators").build_operators(topo, X, p, lean=True)
+    U = _states(ops, 3)
+    bk = pkg("backend").B200Backend(ops, cfg.FlowConditions(flux="hllc"), cfg.SolverOptions(cfl=0.5),
+                                   device_metrics=True)
+    out = {}
+    for name in ("t1", "split4"):
+        pkg("autotune").apply_variant(bk.mesh, name)
+        R, wave = bk.residual(U)
+        F, _ = bk.rate(U)
+        U1, res, flags = bk.step_record(U)
+        out[name] = (R, wave, F, U1, np.array([res])), flags
+    for x, y in zip(out["t1"][0], out["split4"][0]):
+        assert rel(y, x) < TOL
+    assert np.array_equal(out["t1"][1], out["split4"][1])
+
+
+def test_a_lone_large_instance_keeps_the_one_thread_kernel():
+    """Which buckets the exception to the variant table takes (autotune.bucket_context)."""
+    at = pkg("autotune")
+    assert at.bucket_context(1, at.LONE_ELEMENTS + 1, "batch") == "lone"
+    assert at.bucket_context(1, at.LONE_ELEMENTS, "batch") == "batch"
+    assert at.bucket_context(2, 10**6, "batch") == "batch"
+    assert at.bucket_context(1, 10**6, "single") == "single"
+    assert at.variant_for("tri", 3, "lone") == "t1"
