@@ -58,6 +58,7 @@ struct AdjWork {
   double* f2;
   double* norm_partial;  // defect: per-block sum of squares (nullable)
   double* elem_norm;     // defect: per-element sum of squares (nullable)
+  const double* jac;     // the face points' flux Jacobians (k_tile_jac), or null: differentiated here
 };
 
 struct CoordWork {

@@ -17,8 +17,8 @@
 #include "adjoint_dispatch.cuh"
 #include "element.cuh"
 #include "forward_dispatch.cuh"
-#include "split.cuh"
 #include "nozzle_b200.h"
+#include "tile.cuh"
 
 namespace nzb {
 
@@ -52,8 +52,8 @@ static int check_mesh(const nzb_mesh* m) {
   if (m->order < 0 || m->order > MAX_ORDER) return fail("order must lie in 0..3");
   if (m->affine && m->kind != NZB_TRI) return fail("affine geometry is for straight-sided triangles");
   if (m->n_elem <= 0) return fail("mesh has no elements");
-  if (m->split != 0 && m->split != 1 && m->split != SPLIT_T) return fail("split must be 0, 1 or 4 threads per element");
-  if (m->vjp_split != 0 && m->vjp_split != 1 && m->vjp_split != SPLIT_T)
+  if (m->split != 0 && m->split != 1 && m->split != TILE_LANES) return fail("split must be 0, 1 or 4 threads per element");
+  if (m->vjp_split != 0 && m->vjp_split != 1 && m->vjp_split != TILE_LANES)
     return fail("vjp_split must be 0, 1 or 4 threads per element");
   if (!m->area || !m->face_nbr || !m->face_code || !m->face_edge || !m->edge_geo)
     return fail("mesh arrays area/face_nbr/face_code/face_edge/edge_geo are required");
@@ -80,11 +80,11 @@ static int block_threads(int kind, int order) {
 // Elements per block of the forward element kernel: 32 with four threads per
 // element, else one per thread.
 static int element_width(const nzb_mesh& m) {
-  return (m.split == SPLIT_T && m.order > 0) ? SPLIT_EB : block_threads(m.kind, m.order);
+  return (m.split == TILE_LANES && m.order > 0) ? TILE_EB : block_threads(m.kind, m.order);
 }
 // ... and of the adjoint state kernel.
 static int adjoint_width(const nzb_mesh& m) {
-  return (m.vjp_split == SPLIT_T && m.order > 0) ? SPLIT_EB : block_threads(m.kind, m.order);
+  return (m.vjp_split == TILE_LANES && m.order > 0) ? TILE_EB : block_threads(m.kind, m.order);
 }
 // Blocks of the forward element kernel (= norm partial slots of stage 1).
 static int64_t element_blocks(const nzb_mesh& m) { return (m.n_elem + element_width(m) - 1) / element_width(m); }
@@ -522,6 +522,9 @@ struct AdjBatch {
   std::vector<cudaStream_t> bstream;
   std::vector<cudaEvent_t> bdone;
   cudaEvent_t fork = nullptr;
+  // per bucket: room for its face Jacobians, formed at the start of every run (null: a variant
+  // without them, or no memory for them -- then every product differentiates the fluxes itself)
+  std::vector<double*> jac;
   std::map<int, cudaGraphExec_t> graphs;  // key: steps per chunk
 };
 
@@ -536,6 +539,7 @@ static int enqueue_adjoint_step(const AdjBatch& A, size_t b, cudaStream_t st) {
   w.f0 = bf.f0;
   w.f1 = bf.f1;
   w.f2 = bf.f2;
+  w.jac = A.jac[b];
   // stage inputs alternate between two buffers, so no stage reads what it writes
   const double* in[4] = {bf.lam, bf.Y1, bf.Y2, bf.Y1};
   double* outp[4] = {bf.Y1, bf.Y2, bf.Y1, nullptr};
@@ -548,7 +552,7 @@ static int enqueue_adjoint_step(const AdjBatch& A, size_t b, cudaStream_t st) {
   return 0;
 }
 
-static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, cudaStream_t st) {
+static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, bool jac, cudaStream_t st) {
   const nzb_adjoint_buffers& bf = A.buf[b];
   AdjWork w{};
   w.mode = ADJ_DEFECT;
@@ -556,6 +560,7 @@ static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, cudaStream_t st) 
   w.seed = bf.seed;
   w.lam = bf.lam;
   w.elem_norm = A.am.elem_norm + A.offset[b];
+  w.jac = jac ? A.jac[b] : nullptr;
   return dispatch_vjp(A.mesh[b], A.phys[b], w, st);
 }
 
@@ -570,8 +575,15 @@ static int adjoint_graph(AdjBatch& A, int n, cudaGraphExec_t* out) {
   int rc = cuda_check(cudaEventRecord(A.fork, A.stream), "fork record");
   for (size_t b = 0; b < A.mesh.size() && rc == 0; ++b) {
     rc = cuda_check(cudaStreamWaitEvent(A.bstream[b], A.fork, 0), "fork wait");
+    // the defect alone (n = 0) is one product: it differentiates the fluxes itself
+    if (rc == 0 && A.jac[b] && n > 0) {
+      const nzb_mesh& m = A.mesh[b];
+      rc = cuda_check(m.kind == NZB_TRI ? vjp_jac_launch_tri(m, A.phys[b], A.buf[b].U, A.jac[b], A.bstream[b])
+                                        : vjp_jac_launch_quad(m, A.phys[b], A.buf[b].U, A.jac[b], A.bstream[b]),
+                      "face Jacobian launch");
+    }
     for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_adjoint_step(A, b, A.bstream[b]);
-    if (rc == 0) rc = enqueue_adjoint_defect(A, b, A.bstream[b]);
+    if (rc == 0) rc = enqueue_adjoint_defect(A, b, n > 0, A.bstream[b]);
     if (rc == 0) rc = cuda_check(cudaEventRecord(A.bdone[b], A.bstream[b]), "join record");
     if (rc == 0) rc = cuda_check(cudaStreamWaitEvent(A.stream, A.bdone[b], 0), "join wait");
   }
@@ -671,8 +683,8 @@ int nzb_upload_tables(int kind, int order, const double* tables, int64_t n) {
       cuda_check(upload_tables_quad(tables, (size_t)n, off), "table upload (adjoint, quadrilaterals)") ||
       cuda_check(kind == NZB_TRI ? upload_tiles_fwd_tri(order, tables) : upload_tiles_fwd_quad(order, tables),
                  "tile fragment upload") ||
-      cuda_check(kind == NZB_TRI ? prepare_vjp_split_tri(order) : prepare_vjp_split_quad(order),
-                 "adjoint split kernel attributes"))
+      cuda_check(kind == NZB_TRI ? upload_tiles_vjp_tri(order, tables) : upload_tiles_vjp_quad(order, tables),
+                 "adjoint tile fragment upload"))
     return -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -899,7 +911,7 @@ int nzb_stage(const nzb_mesh* mesh, const nzb_physics* phys, const nzb_stage_arg
   return dispatch(*mesh, *phys, w, (cudaStream_t)stream);
 }
 
-int64_t nzb_norm_blocks(int64_t n_elem) { return n_elem <= 0 ? 0 : (n_elem + SPLIT_EB - 1) / SPLIT_EB; }
+int64_t nzb_norm_blocks(int64_t n_elem) { return n_elem <= 0 ? 0 : (n_elem + TILE_EB - 1) / TILE_EB; }
 
 int64_t nzb_element_blocks(const nzb_mesh* mesh) { return mesh ? element_blocks(*mesh) : -1; }
 
@@ -1180,6 +1192,16 @@ int nzb_adjoint_create(int n_buckets, const nzb_mesh* meshes, const nzb_physics*
       nzb_adjoint_destroy(reinterpret_cast<nzb_adjoint*>(A));
       return -1;
     }
+    const nzb_mesh& m = A->mesh[b];
+    const int64_t n = m.vjp_split != TILE_LANES ? 0
+                      : m.kind == NZB_TRI       ? vjp_jac_doubles_tri(m.order, m.n_elem)
+                                                : vjp_jac_doubles_quad(m.order, m.n_elem);
+    double* jac = nullptr;
+    if (n > 0 && cudaMalloc(&jac, sizeof(double) * n) != cudaSuccess) {
+      cudaGetLastError();  // not enough memory: the products work without
+      jac = nullptr;
+    }
+    A->jac.push_back(jac);
   }
   *out = reinterpret_cast<nzb_adjoint*>(A);
   return 0;
@@ -1206,6 +1228,8 @@ int nzb_adjoint_destroy(nzb_adjoint* adjoint) {
   AdjBatch* A = reinterpret_cast<AdjBatch*>(adjoint);
   if (!A) return 0;
   for (auto& kv : A->graphs) cudaGraphExecDestroy(kv.second);
+  for (double* p : A->jac)
+    if (p) cudaFree(p);
   if (A->ev_in) cudaEventDestroy(A->ev_in);
   if (A->ev_out) cudaEventDestroy(A->ev_out);
   if (A->fork) cudaEventDestroy(A->fork);

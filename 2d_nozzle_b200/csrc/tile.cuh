@@ -72,8 +72,20 @@ struct Tile {
   static constexpr int ETA = XI + (K == 1 ? VS : 0);       // quads: [VS] lane values eta_q
   static constexpr int WF = ETA + (K == 1 ? VS : 0);       // lane value: the face point's weight
   static constexpr int COMMON_END = WF + 1;
-  static constexpr int COUNT = COMMON_END + COMMON;
   static constexpr int STAGED = COMMON_END;         // fragments staged by either range
+  // The adjoint kernels' own range [A_PHI, COUNT) (adjoint_tile.cuh): the same tables as it reads them.
+  static constexpr int A_PHI = COMMON_END + COMMON;  // [VT][NS][3] nodes -> phi, w dphi/dxi, w dphi/deta at the points
+  static constexpr int A_TRO = A_PHI + 3 * VT * NS;  // traces, as TRO and TRN
+  static constexpr int A_TRN = A_TRO + 1;
+  static constexpr int A_PT = A_TRN + 1;             // [VS][NT] points -> nodes (phi)
+  static constexpr int A_LF = A_PT + VS * NT;        // [FS][NT] face points -> nodes
+  static constexpr int A_MI = A_LF + FS * NT;        // [NS][NT] tri: M_ref^-1; quads: nodes -> points, Phi^-1
+  static constexpr int A_MT = A_MI + NS * NT;        // quads: [NS][NT], as MT
+  static constexpr int A_WV = A_MT + (K == 1 ? NS * NT : 0);
+  static constexpr int A_XI = A_WV + (K == 1 ? VS : 0);
+  static constexpr int A_ETA = A_XI + (K == 1 ? VS : 0);
+  static constexpr int A_WF = A_ETA + (K == 1 ? VS : 0);
+  static constexpr int COUNT = A_WF + 1;
   // [VS][NT][2 xi, eta] points -> nodes and [FS][NT] face points -> nodes
   static constexpr int vx(int folded, int v, int t, int d) { return (folded ? COMMON_END : 0) + (v * NT + t) * 2 + d; }
   static constexpr int lf(int folded, int fs, int t) { return (folded ? COMMON_END : 0) + VXN + fs * NT + t; }
@@ -219,6 +231,39 @@ std::vector<double> tile_tables(const double* slot) {
   }
   for (int v = 0; v < T::VS; ++v) put_lane(T::WV + v, [&](int l) { return 4 * v + l < NQV ? wv[4 * v + l] : 0.0; });
   put_lane(T::WF, [&](int l) { return pt_of(l) < NQF ? wf[pt_of(l)] : 0.0; });
+
+  // the adjoint range: new layouts of the interpolation, its transpose and the inverse mass, the rest copied
+  for (int vt = 0; vt < T::VT; ++vt)
+    for (int c = 0; c < T::NS; ++c)
+      for (int d = 0; d < 3; ++d)
+        put(T::A_PHI + (vt * T::NS + c) * 3 + d, [&](int k, int j, int l) {
+          const int i = 4 * c + k, q = 4 * (2 * vt + j) + l;
+          return i < NP && q < NQV ? (d == 0 ? phi : d == 1 ? wxi : weta)[i * NQV + q] : 0.0;
+        });
+  for (int v = 0; v < T::VS; ++v)
+    for (int t = 0; t < T::NT; ++t)
+      put(T::A_PT + v * T::NT + t, [&](int k, int j, int l) {
+        const int q = 4 * v + k, i = 4 * (2 * t + j) + l;
+        return q < NQV && i < NP ? phi[i * NQV + q] : 0.0;
+      });
+  for (int c = 0; c < T::NS; ++c)
+    for (int t = 0; t < T::NT; ++t)
+      put(T::A_MI + c * T::NT + t, [&](int k, int j, int l) {
+        const int i = 4 * c + k, q = 4 * (2 * t + j) + l;
+        return i < NP && q < NP ? (double)G[q * NP + i] : 0.0;
+      });
+  auto copy = [&](int to, int from, int n) {
+    for (int k = 0; k < n * 32; ++k) out[to * 32 + k] = out[from * 32 + k];
+  };
+  copy(T::A_TRO, T::TRO, 2);
+  copy(T::A_LF, T::lf(0, 0, 0), T::LFN);
+  if (K == 1) {
+    copy(T::A_MT, T::MT, T::NS * T::NT);
+    copy(T::A_WV, T::WV, T::VS);
+    copy(T::A_XI, T::XI, T::VS);
+    copy(T::A_ETA, T::ETA, T::VS);
+  }
+  copy(T::A_WF, T::WF, 1);
   return out;
 }
 

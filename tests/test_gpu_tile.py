@@ -56,6 +56,35 @@ def test_tiles_agree_with_one_thread(cuda, kind, p, nx, nr):
     assert np.array_equal(out["t1"][1], out["split4"][1])
 
 
+@pytest.mark.parametrize("kind", ["tri", "quad"])
+@pytest.mark.parametrize("p", [1, 2, 3])
+@pytest.mark.parametrize("nx,nr", [s for s in SIZES if s != (160, 97)] + [(72, 100)])
+def test_adjoint_tiles_agree_with_one_thread(cuda, kind, p, nx, nr, monkeypatch):
+    """The product, the rate (both differentiate the fluxes in the kernel) and a run of three RK4 steps
+    (stored face Jacobians) against the one-thread adjoint kernel."""
+    import torch
+
+    ad, cfg, mesh = pkg("adjoint"), pkg("config"), pkg("mesh")
+    topo, xf, rf = mesh.channel_topology(kind, nx=nx, nr=nr)
+    X = mesh.rectangle_coords(xf, rf)
+    X = X + 0.1 / max(nx, nr) * np.sin(7.0 * X[:, ::-1])
+    ops = pkg("operators").build_operators(topo, X, p)
+    U = torch.as_tensor(_states(ops, 4), device="cuda")
+    rng = np.random.default_rng(5)
+    lam, seed = (torch.as_tensor(rng.standard_normal(tuple(U.shape)), device="cuda") for _ in range(2))
+    out = {}
+    for name in ("t1", "split4"):
+        monkeypatch.setenv("NZB_VJP_VARIANT", name)
+        m = ad.AdjointModel(ops, cfg.FlowConditions(flux="ausmup"), cfg.SolverOptions(cfl=0.5))
+        u, la, sd = (ad.to_soa(x) for x in (U, lam, seed))
+        am = ad.AdjointMarch(m, u, sd, 0.5)
+        lam3, rel3, its, _ = am.solve(tolerance=0.0, max_iterations=3, check_interval=3)
+        out[name] = [m.vjp_state(u, la), m.adjoint_rate(u, la, sd), lam3.clone(), torch.tensor([rel3])]
+        assert its == 3
+    for x, y in zip(out["t1"], out["split4"]):
+        assert rel(y.cpu().numpy(), x.cpu().numpy()) < TOL
+
+
 def test_a_lone_large_instance_keeps_the_one_thread_kernel():
     """Which buckets the exception to the variant table takes (autotune.bucket_context)."""
     at = pkg("autotune")
