@@ -246,6 +246,11 @@ class GenUpdateArgs(C.Structure):
         (n, P) for n in ("V", "U0", "F", "wave", "dt", "out", "partial")]
 
 
+class GenRunArgs(C.Structure):
+    _fields_ = [("ssprk3", I32), ("pad", I32), ("dt_factor", C.c_double)] + [
+        (n, P) for n in ("S0", "S1", "S2", "dt", "elem_norm", "fw", "smax", "res", "counters", "share", "means", "scale")]
+
+
 NZB_WALL_PARAMS = 20
 
 
@@ -280,6 +285,7 @@ SIGNATURES = [
     ("nzb_gen_rate", C.c_int, [C.POINTER(GenMesh), C.POINTER(Physics), C.c_int, P, P, P, P, P, P]),
     ("nzb_gen_limit", C.c_int, [C.POINTER(GenMesh), C.POINTER(Physics), P, P, P]),
     ("nzb_gen_update", C.c_int, [C.POINTER(GenMesh), C.POINTER(Physics), C.POINTER(GenUpdateArgs), P]),
+    ("nzb_gen_run", C.c_int, [C.POINTER(GenMesh), C.POINTER(Physics), C.POINTER(GenRunArgs), C.c_int, P]),
     ("nzb_gen_blocks", I64, [C.POINTER(GenMesh)]),
     ("nzb_gen_geometry", C.c_int, [C.POINTER(GenMesh), C.POINTER(GenGeometryArgs), P]),
     ("nzb_gen_superbee", C.c_int, [C.POINTER(GenMesh), C.POINTER(Physics), P, P, P, P, P, P]),

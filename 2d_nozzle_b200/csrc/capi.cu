@@ -851,6 +851,21 @@ int nzb_gen_limit(const nzb_gen_mesh* mesh, const nzb_physics* phys, double* U, 
   return cuda_check(gen_limit_launch(*mesh, *phys, U, counters, (cudaStream_t)stream), "generic limiter launch");
 }
 
+int nzb_gen_run(const nzb_gen_mesh* mesh, const nzb_physics* phys, const nzb_gen_run_args* args, int n_steps,
+                void* stream) {
+  if (check_gen(mesh, phys)) return -1;
+  if (!args || n_steps < 1) return fail("gen_run: null arguments, or n_steps below 1");
+  const nzb_gen_run_args& r = *args;
+  if (!r.S0 || !r.dt || !r.elem_norm || !r.fw || !r.smax || !r.res || (r.ssprk3 && (!r.S1 || !r.S2)))
+    return fail("gen_run: missing array");
+  if (!mesh->grad_x_m || !mesh->grad_y_m || !mesh->face_basis_m || !mesh->elem_area)
+    return fail("gen_run: the mesh lacks the folded operators or the areas");
+  if (phys->limiter != 0 && !mesh->mean_weights) return fail("gen_run: the mesh lacks mean_weights");
+  if (phys->limiter == 2 && (!r.share || !r.means || !r.scale)) return fail("gen_run: the Superbee limiter needs share, means and scale");
+  if (cuda_check(gen_run_launch(*mesh, *phys, r, n_steps, (cudaStream_t)stream), "generic run")) return -1;
+  return nzb_norm_finalize(r.elem_norm, mesh->n_elem, 4.0 * (double)mesh->n_elem * mesh->np, r.res, stream);
+}
+
 int nzb_gen_update(const nzb_gen_mesh* mesh, const nzb_physics* phys, const nzb_gen_update_args* args, void* stream) {
   if (check_gen(mesh, phys)) return -1;
   if (!args || !args->V || !args->F || !args->dt || !args->out || (args->a != 0.0 && !args->U0) ||

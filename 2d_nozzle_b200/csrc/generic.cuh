@@ -14,226 +14,218 @@
 // reference's layout; the state is (E, NP, 4).  The passes follow the
 // reference's compiled path (src/backends/_numba_kernels.py):
 //
-//   k_gen_edge     one thread per edge: both traces at each edge point, the
-//                  Riemann or boundary flux, fw = flux |dX/dsigma| w, the
-//                  edge's largest signal speed;
-//   k_gen_element  one thread per element: the volume term and the gathered
-//                  face terms -- the residual (unfolded operators and the
-//                  reference face basis with the face sign) or the rate
-//                  -M^-1 R (folded operators) -- and the wave-speed sum;
-//   k_gen_limit    one thread per element: the positivity limiter in place
-//                  (mean repair, Lebesgue screen, probe minima at the volume
-//                  points and the element's own face points, closed-form
-//                  density factor, 12-step pressure bisection);
-//   k_gen_update   the local step from the wave sums (stage 1), the stage
-//                  update a U0 + b (V + dt F) and the weighted norm's per-block
-//                  partial sums of stage 1's rate.
+//   k_gen_edge     eight lanes per edge, one per point (in turn past eight): both
+//                  traces, the Riemann or boundary flux, fw = flux |dX/dsigma| w,
+//                  the edge's largest signal speed;
+//   k_gen_element  a warp per element, everything else of a residual, a rate, a
+//                  stage or the limiter alone: the volume states and fluxes (a
+//                  lane per point, through shared memory), the volume term and
+//                  the gathered face terms, the wave-speed sum, the local step,
+//                  the stage update a U0 + b (V + dt F) and the weighted norm's
+//                  element sum, and the positivity limiter (mean repair, Lebesgue
+//                  screen, probe values held in shared memory, 12-step pressure
+//                  bisection).
+//
+// What bounds a stage: the operators are the element's own (7.8 KB for a
+// fourth-order triangle, 34 KB at p = 5), so they are read once, each by one warp, as
+// FP64 mma A fragments: rows are nodes, a k-step four consecutive points of a
+// row (32 contiguous bytes a row), the B operand the four components of the point
+// fluxes (half its columns are unused, which costs nothing where loads decide).
+// With a thread per element instead, each lane walked its own operators: 2 240
+// elements were 18 blocks, 210 us for the element pass alone.  Measured on a B200,
+// a whole stage (all passes, positivity limiter): 2 240 fourth-order triangles
+// 310 -> 23 us, 4 480 curved quadratic quadrilaterals 165 -> 28 us.
 // The flux, boundary and primitive formulas are physics.cuh's, shared with
-// the specialised kernels.  Each element's scratch (its NP x 4 accumulators)
-// is a compile-time-sized array: the kernels are instantiated per NP.
+// the specialised kernels.
 #pragma once
 #include <cstdint>
 
 #include "element.cuh"
+#include "flux.cuh"
 #include "physics.cuh"
 #include "slope.cuh"
+#include "tile.cuh"
 
 namespace nzb {
 
-// The largest number of basis functions an instantiation serves, per bucket.
-__host__ __device__ constexpr int gen_np_bucket(int np) {
-  return np <= 4 ? 4 : np <= 6 ? 6 : np <= 10 ? 10 : np <= 16 ? 16 : np <= 21 ? 21 : np <= 28 ? 28 : 36;
-}
 constexpr int GEN_NP_MAX = 36;
+constexpr int GEN_WARPS = 4;  // elements (warps) of a block
+
+enum { GEN_RESIDUAL = 0, GEN_RATE = 1, GEN_STAGE = 2, GEN_LIMIT = 3 };
+
+struct GenWork {
+  int op, stage, limit;    // limit: the positivity limiter ends the stage
+  const double* V;         // state the rate is evaluated at (the limiter's state)
+  const double* U0;        // step start state (a != 0)
+  double* out;
+  double* wave;            // (E, nullable)
+  const double* fw;        // the edge pass's fluxes and speeds
+  const double* smax;
+  double* dt;
+  double* elem_norm;       // stage 1: the element's weighted squares (nullable)
+  unsigned long long* counters;
+  double dt_factor, a, b;
+};
+
+// Shared doubles of one warp: the state, and the point fluxes or the limiter's probe values.
+struct GenSmem {
+  int np, nqv, nface, nqf;
+  __host__ __device__ int points() const { return nqv + nface * nqf; }
+  __host__ __device__ int scratch() const { return 8 * nqv > 4 * points() ? 8 * nqv : 4 * points(); }
+  __host__ __device__ int warp() const { return 4 * np + scratch(); }
+};
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+__device__ __forceinline__ double warp_min(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w < v ? w : v;
+  }
+  return v;
+}
 
 __global__ void __launch_bounds__(128) k_gen_edge(const nzb_gen_mesh m, const nzb_physics ph, const double* __restrict__ U,
                                                   double* __restrict__ fw, double* __restrict__ smax) {
   const int64_t n_edge = m.n_int + m.n_bnd;
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n_edge) return;
-  const int np = m.np, nqf = m.nqf, nf = m.nface;
-  const bool interior = k < m.n_int;
-  const int64_t le = m.edge_elem[2 * k], re = m.edge_elem[2 * k + 1];
-  const int lf = m.edge_face[2 * k], rf = m.edge_face[2 * k + 1];
-  const int tag = interior ? 0 : m.edge_tag[k - m.n_int];
-  const double* Ul = U + le * np * 4;
-  const double* Ur = U + (interior ? re : le) * np * 4;
+  const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   double best = 0.0;
-  for (int q = 0; q < nqf; ++q) {
-    double UL[4] = {0.0, 0.0, 0.0, 0.0}, UR[4] = {0.0, 0.0, 0.0, 0.0}, F[4];
-    for (int i = 0; i < np; ++i) {
-      const double bl = m.phi_face[(((int64_t)0 * nf + lf) * np + i) * nqf + q];
+  if (k < n_edge) {
+    const int np = m.np, nqf = m.nqf, nf = m.nface;
+    const bool interior = k < m.n_int;
+    const int64_t le = m.edge_elem[2 * k], re = m.edge_elem[2 * k + 1];
+    const int lf = m.edge_face[2 * k], rf = m.edge_face[2 * k + 1];
+    const int tag = interior ? 0 : m.edge_tag[k - m.n_int];
+    const double* Ul = U + le * np * 4;
+    const double* Ur = U + (interior ? re : le) * np * 4;
+    for (int q = threadIdx.x & 7; q < nqf; q += 8) {
+      const double* bl = m.phi_face + (int64_t)lf * np * nqf + q;
+      const double* br = m.phi_face + (int64_t)(nf + rf) * np * nqf + q;
+      double UL[4] = {0.0, 0.0, 0.0, 0.0}, UR[4] = {0.0, 0.0, 0.0, 0.0}, F[4];
+#pragma unroll 4
+      for (int i = 0; i < np; ++i) {
+        const double b = __ldg(bl + i * nqf);
 #pragma unroll
-      for (int s = 0; s < 4; ++s) UL[s] = fma(bl, Ul[i * 4 + s], UL[s]);
+        for (int s = 0; s < 4; ++s) UL[s] = fma(b, __ldg(Ul + i * 4 + s), UL[s]);
+      }
       if (interior) {
-        const double br = m.phi_face[(((int64_t)1 * nf + rf) * np + i) * nqf + q];
+#pragma unroll 4
+        for (int i = 0; i < np; ++i) {
+          const double b = __ldg(br + i * nqf);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) UR[s] = fma(br, Ur[i * 4 + s], UR[s]);
-      }
-    }
-    const double nx = m.edge_normal[(k * nqf + q) * 2], ny = m.edge_normal[(k * nqf + q) * 2 + 1];
-    const double sp = interior ? interface_flux(UL, UR, nx, ny, ph, F) : boundary_flux(tag, UL, nx, ny, ph, ph.p_back, F);
-    best = sp > best ? sp : best;
-    const double scale = m.edge_jac[k * nqf + q] * m.w_face[q];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) fw[(k * nqf + q) * 4 + s] = F[s] * scale;
-  }
-  smax[k] = best;
-}
-
-template <int NPB>
-__global__ void __launch_bounds__(128) k_gen_element(const nzb_gen_mesh m, const nzb_physics ph, int unfolded,
-                                                     const double* __restrict__ U, const double* __restrict__ fw,
-                                                     const double* __restrict__ smax, double* __restrict__ out,
-                                                     double* __restrict__ wave) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.n_elem) return;
-  const int np = m.np, nqv = m.nqv, nqf = m.nqf, nf = m.nface;
-  const double g = ph.gamma;
-  const double* Ue = U + e * np * 4;
-  const double* gx = (unfolded ? m.grad_x : m.grad_x_m) + e * np * nqv;
-  const double* gy = (unfolded ? m.grad_y : m.grad_y_m) + e * np * nqv;
-  double R[NPB][4];
-#pragma unroll
-  for (int i = 0; i < NPB; ++i)
-#pragma unroll
-    for (int s = 0; s < 4; ++s) R[i][s] = 0.0;
-  for (int q = 0; q < nqv; ++q) {
-    double u[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int i = 0; i < NPB; ++i) {
-      if (i < np) {
-        const double b = m.phi_vol[i * nqv + q];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) u[s] = fma(b, Ue[i * 4 + s], u[s]);
-      }
-    }
-    const Prim pr = primitives_fast(u, g);
-    const double F[4] = {pr.rho * pr.vx, pr.rho * pr.vx * pr.vx + pr.p, pr.rho * pr.vx * pr.vy, pr.rho * pr.vx * pr.H};
-    const double G[4] = {pr.rho * pr.vy, pr.rho * pr.vx * pr.vy, pr.rho * pr.vy * pr.vy + pr.p, pr.rho * pr.vy * pr.H};
-#pragma unroll
-    for (int i = 0; i < NPB; ++i) {
-      if (i < np) {
-        const double a = gx[i * nqv + q], b = gy[i * nqv + q];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) R[i][s] -= a * F[s] + b * G[s];
-      }
-    }
-  }
-  double acc = 0.0;
-  for (int f = 0; f < nf; ++f) {
-    const int64_t k = m.face_edge[e * nf + f];
-    const double sg = m.face_sign[e * nf + f];
-    const int sd = m.face_side[e * nf + f];
-    for (int q = 0; q < nqf; ++q) {
-      const double* w = fw + (k * nqf + q) * 4;
-#pragma unroll
-      for (int i = 0; i < NPB; ++i) {
-        if (i < np) {
-          const double b = sg * (unfolded ? m.phi_face[(((int64_t)sd * nf + f) * np + i) * nqf + q]
-                                          : m.face_basis_m[((e * nf + f) * np + i) * nqf + q]);
-#pragma unroll
-          for (int s = 0; s < 4; ++s) R[i][s] = fma(b, w[s], R[i][s]);
+          for (int s = 0; s < 4; ++s) UR[s] = fma(b, __ldg(Ur + i * 4 + s), UR[s]);
         }
       }
-    }
-    acc += smax[k] * m.edge_length[k];
-  }
-  if (wave) wave[e] = acc;
+      const double nx = m.edge_normal[(k * nqf + q) * 2], ny = m.edge_normal[(k * nqf + q) * 2 + 1];
+      const double sp = interior ? lean_interface_flux(UL, UR, nx, ny, ph, F) : boundary_flux(tag, UL, nx, ny, ph, ph.p_back, F);
+      best = sp > best ? sp : best;
+      const double scale = m.edge_jac[k * nqf + q] * m.w_face[q];
 #pragma unroll
-  for (int i = 0; i < NPB; ++i) {
-    if (i < np) {
-#pragma unroll
-      for (int s = 0; s < 4; ++s) out[(e * np + i) * 4 + s] = unfolded ? R[i][s] : -R[i][s];
+      for (int s = 0; s < 4; ++s) fw[(k * nqf + q) * 4 + s] = F[s] * scale;
     }
   }
-}
-
-// The minimum density and pressure of ubar + theta (u - ubar) over the element's probe points: the
-// volume points, then its own trace at each face point (src/backends/_numba_kernels.py:856-924).
-template <int NPB>
-__device__ void gen_probe_minima(const nzb_gen_mesh& m, const double* Ue, const double (&ub)[4], double theta,
-                                 const int* fside, double g, double& rmin, double& pmin) {
-  const int np = m.np, nqv = m.nqv, nqf = m.nqf, nf = m.nface;
-  double rm = 1e300, pm = 1e300;
-  const int npt = nqv + nf * nqf;
-  for (int pt = 0; pt < npt; ++pt) {
-    double u[4] = {0.0, 0.0, 0.0, 0.0};
-    const double* basis;
-    int stride;
-    if (pt < nqv) {
-      basis = m.phi_vol + pt;
-      stride = nqv;
-    } else {
-      const int f = (pt - nqv) / nqf, q = (pt - nqv) - f * nqf;
-      basis = m.phi_face + (((int64_t)fside[f] * nf + f) * np) * nqf + q;
-      stride = nqf;
-    }
 #pragma unroll
-    for (int i = 0; i < NPB; ++i) {
-      if (i < np) {
-        const double b = basis[i * stride];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) u[s] = fma(b, Ue[i * 4 + s], u[s]);
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) u[s] = ub[s] + theta * (u[s] - ub[s]);
-    rm = u[0] < rm ? u[0] : rm;
-    const double r = u[0] > 1e-300 ? u[0] : 1e-300;
-    const double pp = (g - 1.0) * (u[3] - 0.5 * (u[1] * u[1] + u[2] * u[2]) / r);
-    pm = pp < pm ? pp : pm;
+  for (int o = 4; o > 0; o >>= 1) {
+    const double v = __shfl_xor_sync(0xffffffffu, best, o);
+    best = v > best ? v : best;
   }
-  rmin = rm;
-  pmin = pm;
+  if (k < n_edge && (threadIdx.x & 7) == 0) smax[k] = best;
 }
 
 // The positivity limiter of one element in place (src/backends/_numba_kernels.py:927-1093;
-// src/spatial/limiter.py:103-243): an element it leaves alone is not rewritten.
-template <int NPB>
-__device__ __forceinline__ void gen_limit_element(const nzb_gen_mesh& m, const nzb_physics& ph, int64_t e,
-                                                  double* __restrict__ Ue, int& scaled, int& repaired) {
-  const int np = m.np, nf = m.nface;
+// src/spatial/limiter.py:103-243), by its warp: su the (NP, 4) state, sp room for the probe values.
+// Every decision is the same on every lane.
+__device__ __forceinline__ void gen_limit_warp(const nzb_gen_mesh& m, const nzb_physics& ph, int64_t e, double* su,
+                                               double* sp, int& scaled, int& repaired) {
+  const int lane = threadIdx.x & 31;
+  const int np = m.np, nqv = m.nqv, nqf = m.nqf, nf = m.nface;
   const double g = ph.gamma, g1 = g - 1.0, lam = ph.lebesgue;
   double ub[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i = lane; i < np; i += 32) {
+    const double w = __ldg(m.mean_weights + e * np + i);
 #pragma unroll
-  for (int i = 0; i < NPB; ++i) {
-    if (i < np) {
-      const double w = m.mean_weights[e * np + i];
-#pragma unroll
-      for (int s = 0; s < 4; ++s) ub[s] = fma(w, Ue[i * 4 + s], ub[s]);
-    }
+    for (int s = 0; s < 4; ++s) ub[s] = fma(w, su[i * 4 + s], ub[s]);
   }
+#pragma unroll
+  for (int s = 0; s < 4; ++s) ub[s] = warp_sum(ub[s]);
   const double rho_new = ub[0] > ph.rho_floor ? ub[0] : ph.rho_floor;
   const double e_min = ph.p_floor / g1 + 0.5 * (ub[1] * ub[1] + ub[2] * ub[2]) / rho_new;
   const double rhoE_new = ub[3] > e_min ? ub[3] : e_min;
   const double d0 = rho_new - ub[0], d3 = rhoE_new - ub[3];
   if (d0 != 0.0 || d3 != 0.0) {
-    for (int i = 0; i < np; ++i) {
-      Ue[i * 4] += d0;
-      Ue[i * 4 + 3] += d3;
+    for (int i = lane; i < np; i += 32) {
+      su[i * 4] += d0;
+      su[i * 4 + 3] += d3;
     }
     ub[0] = rho_new;
     ub[3] = rhoE_new;
     repaired = 1;
+    __syncwarp();
   }
   const double pbar = g1 * (ub[3] - 0.5 * (ub[1] * ub[1] + ub[2] * ub[2]) / ub[0]);
   double eps_r = ph.lim_fraction * ub[0], eps_p = ph.lim_fraction * pbar;
   eps_r = eps_r < 0.5 * ph.rho_floor ? 0.5 * ph.rho_floor : eps_r;
   eps_p = eps_p < 0.5 * ph.p_floor ? 0.5 * ph.p_floor : eps_p;
   double dv[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = 0; i < np; ++i)
+  for (int i = lane; i < np; i += 32)
 #pragma unroll
-    for (int s = 0; s < 4; ++s) dv[s] = fmax(dv[s], fabs(Ue[i * 4 + s] - ub[s]));
+    for (int s = 0; s < 4; ++s) dv[s] = fmax(dv[s], fabs(su[i * 4 + s] - ub[s]));
+#pragma unroll
+  for (int s = 0; s < 4; ++s) dv[s] = warp_max(dv[s]);
   const double rho_lo = ub[0] - lam * dv[0];
   if (rho_lo >= eps_r) {
     const double m_hi = sqrt(ub[1] * ub[1] + ub[2] * ub[2]) + lam * sqrt(dv[1] * dv[1] + dv[2] * dv[2]);
     if (g1 * (ub[3] - lam * dv[3] - 0.5 * m_hi * m_hi / rho_lo) >= eps_p) return;
   }
-  int fside[8];
-  for (int f = 0; f < nf; ++f) fside[f] = m.face_side[e * nf + f];
+  // the probe values: the volume points, then the element's own trace at each face point; a lane
+  // writes and reads its own points only
+  const int npt = nqv + nf * nqf;
+  for (int pt = lane; pt < npt; pt += 32) {
+    const double* basis = m.phi_vol + pt;
+    int stride = nqv;
+    if (pt >= nqv) {
+      const int f = (pt - nqv) / nqf, q = (pt - nqv) - f * nqf;
+      basis = m.phi_face + ((int64_t)(m.face_side[e * nf + f] * nf + f) * np) * nqf + q;
+      stride = nqf;
+    }
+    double u[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = 0; i < np; ++i) {
+      const double b = __ldg(basis + i * stride);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) u[s] = fma(b, su[i * 4 + s], u[s]);
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) sp[pt * 4 + s] = u[s];
+  }
+  // the smallest density and pressure of ubar + theta (u - ubar) over the points
+  auto minima = [&](double theta, double& rmin, double& pmin) {
+    double rm = 1e300, pm = 1e300;
+    for (int pt = lane; pt < npt; pt += 32) {
+      double u[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) u[s] = ub[s] + theta * (sp[pt * 4 + s] - ub[s]);
+      rm = u[0] < rm ? u[0] : rm;
+      const double r = u[0] > 1e-300 ? u[0] : 1e-300;
+      const double pp = g1 * (u[3] - 0.5 * (u[1] * u[1] + u[2] * u[2]) / r);
+      pm = pp < pm ? pp : pm;
+    }
+    rmin = warp_min(rm);
+    pmin = warp_min(pm);
+  };
   double rmin, pmin;
-  gen_probe_minima<NPB>(m, Ue, ub, 1.0, fside, g, rmin, pmin);
+  minima(1.0, rmin, pmin);
   if (!(rmin < eps_r) && !(pmin < eps_p)) return;
   double theta = 1.0;
   if (rmin < eps_r) {
@@ -241,30 +233,29 @@ __device__ __forceinline__ void gen_limit_element(const nzb_gen_mesh& m, const n
     theta = gap <= 0.0 ? 0.0 : (ub[0] - eps_r) / gap;
     theta = theta < 0.0 ? 0.0 : (theta > 1.0 ? 1.0 : theta);
   }
-  double rr, ph_;
-  gen_probe_minima<NPB>(m, Ue, ub, theta, fside, g, rr, ph_);
-  if (ph_ < eps_p) {
+  minima(theta, rmin, pmin);
+  if (pmin < eps_p) {
     double lo = 0.0, hi = theta;
     for (int it = 0; it < ph.lim_steps; ++it) {
       const double mid = 0.5 * (lo + hi);
-      double pm;
-      gen_probe_minima<NPB>(m, Ue, ub, mid, fside, g, rr, pm);
-      if (pm >= eps_p)
+      minima(mid, rmin, pmin);
+      if (pmin >= eps_p)
         lo = mid;
       else
         hi = mid;
     }
     theta = lo;
   }
-  for (int i = 0; i < np; ++i)
+  for (int i = lane; i < np; i += 32)
 #pragma unroll
-    for (int s = 0; s < 4; ++s) Ue[i * 4 + s] = ub[s] + theta * (Ue[i * 4 + s] - ub[s]);
+    for (int s = 0; s < 4; ++s) su[i * 4 + s] = ub[s] + theta * (su[i * 4 + s] - ub[s]);
   scaled = 1;
 }
 
 __device__ __forceinline__ void gen_count(unsigned long long* counters, int scaled, int repaired) {
   if (counters) {
-    const int ns = __syncthreads_count(scaled), nr = __syncthreads_count(repaired);
+    const bool first = (threadIdx.x & 31) == 0;
+    const int ns = __syncthreads_count(first && scaled), nr = __syncthreads_count(first && repaired);
     if (threadIdx.x == 0) {
       if (ns) atomicAdd(counters + 0, (unsigned long long)ns);
       if (nr) atomicAdd(counters + 1, (unsigned long long)nr);
@@ -272,14 +263,148 @@ __device__ __forceinline__ void gen_count(unsigned long long* counters, int scal
   }
 }
 
-// The positivity limiter in place, one thread per element.
-template <int NPB>
-__global__ void __launch_bounds__(128) k_gen_limit(const nzb_gen_mesh m, const nzb_physics ph, double* __restrict__ U,
-                                                   unsigned long long* counters) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// MT: tiles of eight nodes.
+template <int MT>
+__global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_element(const nzb_gen_mesh m, const nzb_physics ph, const GenWork w) {
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x & 31, l = lane & 3, n = lane >> 2;
+  const int np = m.np, nqv = m.nqv, nqf = m.nqf, nf = m.nface;
+  const GenSmem L{np, nqv, nf, nqf};
+  double* const su = smem + (threadIdx.x >> 5) * L.warp();
+  double* const sp = su + 4 * np;
+  const int64_t e = (int64_t)blockIdx.x * GEN_WARPS + (threadIdx.x >> 5);
   int scaled = 0, repaired = 0;
-  if (e < m.n_elem) gen_limit_element<NPB>(m, ph, e, U + e * m.np * 4, scaled, repaired);
-  gen_count(counters, scaled, repaired);
+  if (e < m.n_elem) {
+    const int64_t base = e * np * 4;
+    for (int k = lane; k < np * 4; k += 32) su[k] = w.V[base + k];
+    __syncwarp();
+    if (w.op != GEN_LIMIT) {
+      const bool unfolded = w.op == GEN_RESIDUAL;
+      const double g = ph.gamma;
+      // face f's edge, sign and side in lane f
+      int64_t ke = 0;
+      double sg = 0.0, speed = 0.0;
+      int sd = 0;
+      if (lane < nf) {
+        ke = m.face_edge[e * nf + lane];
+        sg = m.face_sign[e * nf + lane];
+        sd = m.face_side[e * nf + lane];
+        speed = w.smax[ke] * m.edge_length[ke];
+      }
+      // ---- volume states and fluxes, a lane per point
+      for (int q = lane; q < nqv; q += 32) {
+        double u[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+        for (int i = 0; i < np; ++i) {
+          const double b = __ldg(m.phi_vol + i * nqv + q);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) u[s] = fma(b, su[i * 4 + s], u[s]);
+        }
+        const Prim pr = primitives_fast(u, g);
+        double* F = sp + q * 8;
+        F[0] = pr.rho * pr.vx;
+        F[1] = pr.rho * pr.vx * pr.vx + pr.p;
+        F[2] = pr.rho * pr.vx * pr.vy;
+        F[3] = pr.rho * pr.vx * pr.H;
+        F[4] = pr.rho * pr.vy;
+        F[5] = pr.rho * pr.vx * pr.vy;
+        F[6] = pr.rho * pr.vy * pr.vy + pr.p;
+        F[7] = pr.rho * pr.vy * pr.H;
+      }
+      __syncwarp();
+      // ---- acc[i][s] = sum_q (gx F + gy G) - sum_fq basis sign fw: A rows are nodes 8 mt + lane / 4,
+      // a k-step four points, B columns the components (4..7 zero)
+      double acc[MT][2];
+#pragma unroll
+      for (int t = 0; t < MT; ++t) acc[t][0] = acc[t][1] = 0.0;
+      const double* gx = (unfolded ? m.grad_x : m.grad_x_m) + e * np * nqv;
+      const double* gy = (unfolded ? m.grad_y : m.grad_y_m) + e * np * nqv;
+#pragma unroll 2
+      for (int q0 = 0; q0 < nqv; q0 += 4) {
+        const int q = q0 + l;
+        const bool col = n < 4 && q < nqv;
+        const double bF = col ? sp[q * 8 + n] : 0.0, bG = col ? sp[q * 8 + 4 + n] : 0.0;
+        double ax[MT], ay[MT];
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          const int i = 8 * t + n;
+          const bool in = i < np && q < nqv;
+          ax[t] = in ? __ldg(gx + i * nqv + q) : 0.0;
+          ay[t] = in ? __ldg(gy + i * nqv + q) : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          mma(acc[t], ax[t], bF);
+          mma(acc[t], ay[t], bG);
+        }
+      }
+      const int nfq = nf * nqf;
+#pragma unroll 2
+      for (int k0 = 0; k0 < nfq; k0 += 4) {
+        const int kk = k0 + l, f = kk < nfq ? kk / nqf : 0, q = kk - f * nqf;
+        const int64_t k = __shfl_sync(0xffffffffu, ke, f);
+        const double sign = __shfl_sync(0xffffffffu, sg, f);
+        const int side = __shfl_sync(0xffffffffu, sd, f);
+        const double bw = n < 4 && kk < nfq ? -sign * w.fw[(k * nqf + q) * 4 + n] : 0.0;
+        const double* basis = unfolded ? m.phi_face + ((int64_t)(side * nf + f) * np) * nqf + q
+                                       : m.face_basis_m + ((e * nf + f) * np) * nqf + q;
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          const int i = 8 * t + n;
+          mma(acc[t], i < np && kk < nfq ? __ldg(basis + i * nqf) : 0.0, bw);
+        }
+      }
+      double wave = 0.0;
+      for (int f = 0; f < nf; ++f) wave += __shfl_sync(0xffffffffu, speed, f);
+      if (w.wave && lane == 0) w.wave[e] = wave;
+      // node 8 t + lane / 4, components 2 l and 2 l + 1 (l < 2)
+      if (w.op != GEN_STAGE) {
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          const int i = 8 * t + n;
+          if (l < 2 && i < np) {
+            su[i * 4 + 2 * l] = unfolded ? -acc[t][0] : acc[t][0];
+            su[i * 4 + 2 * l + 1] = unfolded ? -acc[t][1] : acc[t][1];
+          }
+        }
+      } else {
+        double d;
+        if (w.stage == 1) {
+          d = w.dt_factor * 2.0 * m.elem_area[e] / (wave < FLOOR ? FLOOR : wave);
+          if (lane == 0) w.dt[e] = d;
+        } else {
+          d = w.dt[e];
+        }
+        double sq = 0.0;
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          const int i = 8 * t + n;
+          if (l < 2 && i < np) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const int k = i * 4 + 2 * l + c;
+              const double f = acc[t][c], v = su[k];
+              const double r = f * ph.norm_w[2 * l + c];
+              sq = fma(r, r, sq);
+              su[k] = w.a == 0.0 ? v + d * f : w.a * w.U0[base + k] + w.b * (v + d * f);
+            }
+          }
+        }
+        if (w.elem_norm) {
+          sq = warp_sum(sq);
+          if (lane == 0) w.elem_norm[e] = sq;
+        }
+      }
+      __syncwarp();
+    }
+    if (w.op == GEN_LIMIT || (w.op == GEN_STAGE && w.limit)) {
+      gen_limit_warp(m, ph, e, su, sp, scaled, repaired);
+      __syncwarp();
+    }
+    for (int k = lane; k < np * 4; k += 32) w.out[base + k] = su[k];
+  }
+  if (w.op == GEN_LIMIT || w.op == GEN_STAGE) gen_count(w.counters, scaled, repaired);
 }
 
 // The Superbee TVB slope limiter (src/spatial/limiter.py:246-429) on the generic path, in the
@@ -327,50 +452,53 @@ __global__ void __launch_bounds__(1024) k_gen_lim_scale(const double* __restrict
   }
 }
 
-template <int NPB>
-__global__ void __launch_bounds__(128) k_gen_superbee(const nzb_gen_mesh m, const nzb_physics ph,
-                                                      double* __restrict__ U, const double* __restrict__ means,
-                                                      const double* __restrict__ scale,
-                                                      const double* __restrict__ share,
-                                                      unsigned long long* counters) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_superbee(const nzb_gen_mesh m, const nzb_physics ph,
+                                                                 double* __restrict__ U, const double* __restrict__ means,
+                                                                 const double* __restrict__ scale,
+                                                                 const double* __restrict__ share,
+                                                                 unsigned long long* counters) {
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x & 31;
+  const int np = m.np, nf = m.nface, nqf = m.nqf;
+  const GenSmem L{np, m.nqv, nf, nqf};
+  double* const su = smem + (threadIdx.x >> 5) * L.warp();
+  double* const sp = su + 4 * np;
+  const int64_t e = (int64_t)blockIdx.x * GEN_WARPS + (threadIdx.x >> 5);
   int scaled = 0, repaired = 0;
   if (e < m.n_elem) {
-    const int np = m.np, nf = m.nface, nqf = m.nqf;
-    double* Ue = U + e * np * 4;
-    double ub[4], sc[4];
+    for (int k = lane; k < np * 4; k += 32) su[k] = U[e * np * 4 + k];
+    __syncwarp();
+    // the own traces at the face points, a lane per point
+    for (int pt = lane; pt < nf * nqf; pt += 32) {
+      const int f = pt / nqf, q = pt - f * nqf;
+      const double* pf = m.phi_face + (int64_t)(m.face_side[e * nf + f] * nf + f) * np * nqf + q;
+      double tr[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int i = 0; i < np; ++i) {
+        const double c = __ldg(pf + i * nqf);
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      ub[s] = means[e * 4 + s];
-      sc[s] = scale[s];
-    }
-    const double sh = share[e];
-    double wsum = 0.0;
-    for (int q = 0; q < nqf; ++q) wsum += m.w_face[q];
-    double theta = 1.0;
-    for (int f = 0; f < nf; ++f) {
-      const int64_t k = m.face_edge[e * nf + f];
-      if (k >= m.n_int) continue;  // a boundary face is not limited against
-      const int64_t a0 = m.edge_elem[2 * k], a1 = m.edge_elem[2 * k + 1];
-      const int64_t nb = a0 == e ? a1 : a0;
-      const int side = m.face_side[e * nf + f];
-      const double* pf = m.phi_face + (int64_t)(side * nf + f) * np * nqf;
-      double tm[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int q = 0; q < nqf; ++q) {
-        double tr[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = 0; i < np; ++i) {
-          const double c = pf[i * nqf + q];
-#pragma unroll
-          for (int s = 0; s < 4; ++s) tr[s] = fma(c, Ue[i * 4 + s], tr[s]);
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s) tm[s] = fma(m.w_face[q], tr[s], tm[s]);
+        for (int s = 0; s < 4; ++s) tr[s] = fma(c, su[i * 4 + s], tr[s]);
       }
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const double d = tm[s] / wsum - ub[s];
-        const double a = means[nb * 4 + s] - ub[s];
-        const bool quiet = fabs(d) <= 1e-12 || fabs(d) <= ph.tvb_constant * sh * sc[s];
+      for (int s = 0; s < 4; ++s) sp[pt * 4 + s] = tr[s];
+    }
+    __syncwarp();
+    // a lane per face and component
+    double theta = 1.0;
+    const int f = lane >> 2, s = lane & 3;
+    if (f < nf) {
+      const int64_t k = m.face_edge[e * nf + f];
+      if (k < m.n_int) {  // a boundary face is not limited against
+        const int64_t a0 = m.edge_elem[2 * k], a1 = m.edge_elem[2 * k + 1];
+        const int64_t nb = a0 == e ? a1 : a0;
+        double wsum = 0.0, tm = 0.0;
+        for (int q = 0; q < nqf; ++q) {
+          wsum += m.w_face[q];
+          tm = fma(m.w_face[q], sp[(f * nqf + q) * 4 + s], tm);
+        }
+        const double ub = means[e * 4 + s];
+        const double d = tm / wsum - ub;
+        const double a = means[nb * 4 + s] - ub;
+        const bool quiet = fabs(d) <= 1e-12 || fabs(d) <= ph.tvb_constant * share[e] * scale[s];
         if (!quiet) {
           double tf = superbee2(a, d) / d;
           tf = tf < 0.0 ? 0.0 : (tf > 1.0 ? 1.0 : tf);
@@ -378,15 +506,19 @@ __global__ void __launch_bounds__(128) k_gen_superbee(const nzb_gen_mesh m, cons
         }
       }
     }
+    theta = warp_min(theta);
     bool changed = false;
-    for (int i = 0; i < np; ++i)
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const double v = ub[s] + theta * (Ue[i * 4 + s] - ub[s]);
-        changed |= v != Ue[i * 4 + s];
-        Ue[i * 4 + s] = v;
-      }
-    gen_limit_element<NPB>(m, ph, e, Ue, scaled, repaired);
+    for (int k = lane; k < np * 4; k += 32) {
+      const double ub = means[e * 4 + (k & 3)];
+      const double v = ub + theta * (su[k] - ub);
+      changed |= v != su[k];
+      su[k] = v;
+    }
+    changed = __any_sync(0xffffffffu, changed);
+    __syncwarp();
+    gen_limit_warp(m, ph, e, su, sp, scaled, repaired);
+    __syncwarp();
+    for (int k = lane; k < np * 4; k += 32) U[e * np * 4 + k] = su[k];
     scaled |= changed ? 1 : 0;
   }
   gen_count(counters, scaled, repaired);

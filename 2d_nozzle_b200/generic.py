@@ -4,9 +4,9 @@
 what the specialised kernels are instantiated for (straight-sided elements of
 order 0..3).  It runs the ``nzb_gen_*`` kernels (csrc/generic.cuh) on the
 reference's own per-element operators (src/spatial/operators.py:139-206),
-uploaded once in the reference's layout: an edge pass and an element pass per
-rate, the positivity limiter in place, the SSP-RK3 / forward-Euler stages with
-the local step and the weighted norm -- the reference's compiled step
+uploaded once in the reference's layout: per SSP-RK3 / forward-Euler stage an
+edge pass and an element pass that ends with the local step, the update, the
+weighted norm and the limiter -- the reference's compiled step
 (src/backends/numba_backend.py:283-337) on the GPU.  The interface is the
 reference's ``Backend`` (src/backends/base.py:81-201), as ``B200Backend``'s.
 
@@ -120,11 +120,9 @@ class GenericB200Backend(B200Backend):
         z = lambda n: torch.zeros(n, dtype=torch.float64, device=dev)  # noqa: E731
         n = E * NP * 4
         self._S = [z(n) for _ in range(3)]
-        self._F = [z(n) for _ in range(3)]
         self._wave, self._dt = z(E), z(E)
         self._fw, self._smax = z(self.n_edge * NQF * 4), z(self.n_edge)
-        self._nb = int(self.lib.nzb_gen_blocks(self._gm))
-        self._partial = z(self._nb)
+        self._elem_norm = z(E)
         self._res = z(1)
         self._counters = torch.zeros(2, dtype=torch.int64, device=dev)
         self._minv = self._arr["inv_mass"].view(E, NP, NP) if device_metrics else None
@@ -207,19 +205,6 @@ class GenericB200Backend(B200Backend):
         else:
             capi.check(self.lib.nzb_gen_limit(self._gm, self._phys_ref, t.data_ptr(), self._counters.data_ptr(),
                                               self._stream), "nzb_gen_limit")
-
-    def _update(self, stage, V, U0, F, out, a=0.0, b=1.0):
-        args = capi.GenUpdateArgs()
-        args.stage = stage
-        args.dt_factor = self.positivity_scale() * _step_coefficient(self.ops.ref.order, self.opts.cfl, self.scheme)
-        args.a, args.b = a, b
-        args.V, args.F, args.wave, args.dt, args.out = (x.data_ptr() for x in (V, F, self._wave, self._dt, out))
-        args.U0 = U0.data_ptr() if U0 is not None else None
-        args.partial = self._partial.data_ptr() if stage == 1 else None
-        capi.check(self.lib.nzb_gen_update(self._gm, self._phys_ref, C.byref(args), self._stream), "nzb_gen_update")
-        if stage == 1:
-            capi.check(self.lib.nzb_norm_finalize(self._partial.data_ptr(), self._nb, 4.0 * self.E * self.NP,
-                                                  self._res.data_ptr(), self._stream), "nzb_norm_finalize")
 
     # -- primitives -----------------------------------------------------------
     def _eval(self, U, unfolded):
@@ -332,26 +317,20 @@ class GenericB200Backend(B200Backend):
 
     # -- the march ---------------------------------------------------------------
     def run_device(self, n_steps: int, scheme: str | None = None) -> None:
-        """Advance the device-resident state (``self._S[0]``) by ``n_steps``: per stage a rate (edge and element
-        passes), the update and the limiter in place, as the reference's fused step orders them."""
+        """Advance the device-resident state (``self._S[0]``) by ``n_steps``: per stage an edge pass and an
+        element pass that ends with the update and the limiter (``nzb_gen_run``)."""
+        if int(n_steps) < 1:
+            return
         scheme = scheme or self.scheme
-        S0, S1, S2 = self._S
-        F0, F1, F2 = self._F
-        for _ in range(int(n_steps)):
-            self._rate_into(S0, F0)
-            if scheme == "euler":
-                self._update(1, S0, None, F0, S1)
-                self._limit_into(S1)
-                S0.copy_(S1)
-                continue
-            self._update(1, S0, None, F0, S2)
-            self._limit_into(S2)
-            self._rate_into(S2, F1)
-            self._update(2, S2, S0, F1, S1, 0.75, 0.25)
-            self._limit_into(S1)
-            self._rate_into(S1, F2)
-            self._update(3, S1, S0, F2, S0, 1.0 / 3.0, 2.0 / 3.0)
-            self._limit_into(S0)
+        a = capi.GenRunArgs()
+        a.ssprk3 = 0 if scheme == "euler" else 1
+        a.dt_factor = self.positivity_scale() * _step_coefficient(self.ops.ref.order, self.opts.cfl, self.scheme)
+        a.S0, a.S1, a.S2 = (t.data_ptr() for t in self._S)
+        a.dt, a.elem_norm, a.fw, a.smax, a.res, a.counters = (
+            t.data_ptr() for t in (self._dt, self._elem_norm, self._fw, self._smax, self._res, self._counters))
+        if self.opts.limiter == "superbee":
+            a.share, a.means, a.scale = (t.data_ptr() for t in (self._share, self._means, self._scale))
+        capi.check(self.lib.nzb_gen_run(self._gm, self._phys_ref, C.byref(a), int(n_steps), self._stream), "nzb_gen_run")
 
     def run(self, U, n_steps: int, scheme: str):
         """Advance ``n_steps`` steps; returns a fresh ``(U, residual of the last step)``."""

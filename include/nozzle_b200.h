@@ -553,6 +553,29 @@ int64_t nzb_gen_blocks(const nzb_gen_mesh* mesh);
 int nzb_gen_superbee(const nzb_gen_mesh* mesh, const nzb_physics* phys, double* U, const double* share,
                      double* means, double* scale, unsigned long long* counters, void* stream);
 
+/* n_steps SSP-RK3 (or forward Euler) steps of the state S0 in place, each stage an edge pass and an
+ * element pass that ends with the stage update and the mesh's limiter (phys->limiter: 0 none, 1
+ * positivity, 2 Superbee then positivity): the reference's compiled step (src/backends/
+ * numba_backend.py:283-337).  res receives the weighted RMS of the last step's first rate. */
+typedef struct {
+  int32_t ssprk3, pad;
+  double dt_factor;
+  double* S0;                     /* (E, NP, 4) */
+  double* S1;                     /* scratch states (ssprk3) */
+  double* S2;
+  double* dt;                     /* (E) */
+  double* elem_norm;              /* (E) scratch */
+  double* fw;                     /* (n_edge, NQF, 4) scratch of the edge pass */
+  double* smax;                   /* (n_edge) */
+  double* res;                    /* (1) */
+  unsigned long long* counters;   /* 2 x uint64, nullable: scaled and repaired elements, accumulated */
+  const double* share;            /* Superbee: as nzb_gen_superbee's */
+  double* means;
+  double* scale;
+} nzb_gen_run_args;
+int nzb_gen_run(const nzb_gen_mesh* mesh, const nzb_physics* phys, const nzb_gen_run_args* args, int n_steps,
+                void* stream);
+
 /* The coordinate-dependent operators of the generic path built on the device
  * from the node coordinates, for any order and geometry order (the
  * coordinate part of build_operators, src/spatial/operators.py:209-342): per
