@@ -70,13 +70,15 @@ class AdjointModel:
         self.phys = physics_struct(flow, opts, ops.ref)
         self.dgs = np.ascontiguousarray(face_tangent_table(ops.ref).ravel())  # host: passed by value to the kernel
         self.elem_nodes = np.ascontiguousarray(np.asarray(ops.topology.elem_nodes)[:, : self.NV])
-        self.elem_nodes_t = torch.as_tensor(self.elem_nodes, device=self.device)
+        self.elem_nodes_t = torch.as_tensor(self.elem_nodes.astype(np.int64), device=self.device)
         self.X0 = torch.as_tensor(np.asarray(ops.node_coords, float), device=self.device)
         # per-block partial sums of the defect: room for the most blocks any variant launches (32 elements
         # per block); slots past the launched blocks stay zero
         self._partial = torch.zeros(max(int(self.lib.nzb_element_blocks(self.mesh.c_ref)), (self.E + 31) // 32),
                                     dtype=torch.float64, device=self.device)
         self._other = (None, None)  # (coordinates, DeviceMesh) of the last mesh built away from X0
+        self._n_node = int(self.elem_nodes.max()) + 1
+        self._node_items = None  # element vertices by node, for the coordinate product's sums
 
     @property
     def stream(self):
@@ -91,10 +93,29 @@ class AdjointModel:
 
     def mesh_at(self, X):
         """The device mesh at node coordinates X (this model's own when X is its base coordinates)."""
-        # coordinates from the torch and NumPy contour code can differ in the last bit
-        if X is None or (X.shape == self.X0.shape and torch.allclose(X.detach().to(self.device), self.X0,
-                                                                     rtol=1e-14, atol=1e-15)):
-            return self.mesh
+        return self._at(X, None)[0]
+
+    def _at(self, X, p_back):
+        """(device mesh at X, back pressure as a float or None): the two values a launch needs from the
+        device, read in one copy."""
+        on_device = torch.is_tensor(p_back) and p_back.is_cuda
+        pb = None if p_back is None or on_device else float(p_back)
+        if X is None or (X.shape == self.X0.shape and X.dtype != self.X0.dtype):
+            same = X is None or torch.allclose(X.detach().to(self.device), self.X0, rtol=1e-14, atol=1e-15)
+            return (self.mesh if same else self._mesh_away(X)), float(p_back) if on_device else pb
+        if X.shape == self.X0.shape:
+            # coordinates from the torch and NumPy contour code can differ in the last bit
+            Xd = X.detach().to(self.device).contiguous()
+            got = torch.zeros(2, dtype=torch.float64, device=self.device)
+            capi.check(self.lib.nzb_all_close(Xd.data_ptr(), self.X0.data_ptr(), Xd.numel(), 1e-14, 1e-15, got.data_ptr(),
+                                              self.stream), "nzb_all_close")
+            if on_device:
+                got[1:].copy_(p_back.detach().reshape(1))
+            far, value = got.tolist()
+            return (self._mesh_away(X) if far else self.mesh), value if on_device else pb
+        return self._mesh_away(X), float(p_back) if on_device else pb
+
+    def _mesh_away(self, X):
         # the metric terms at X are rebuilt on the device (nzb_geometry); the connectivity is this mesh's
         Xd = X.detach().to(device=self.device, dtype=torch.float64)
         if self._other[0] is None or not torch.equal(self._other[0], Xd):
@@ -108,21 +129,39 @@ class AdjointModel:
 
     def verts(self, X):
         """(2 NV, E) vertex coordinates of every element."""
-        Xe = X.detach().to(self.device)[self.elem_nodes_t]  # (E, NV, 2)
-        return torch.cat([Xe[:, :, 0].T, Xe[:, :, 1].T], 0).contiguous()
+        Xd = X.detach().to(device=self.device, dtype=torch.float64).contiguous()
+        if Xd.ndim != 2 or Xd.shape[1] != 2 or Xd.shape[0] < self._n_node:
+            raise IndexError(f"node coordinates have shape {tuple(Xd.shape)}; the elements use {self._n_node} nodes")
+        out = torch.empty((2 * self.NV, self.E), dtype=torch.float64, device=self.device)
+        capi.check(self.lib.nzb_element_vertices(Xd.data_ptr(), self.elem_nodes_t.data_ptr(), self.E, self.NV,
+                                                 out.data_ptr(), self.stream), "nzb_element_vertices")
+        return out
+
+    def _node_sums(self, gvert, n_node):
+        """(2, NV, E) element-vertex values summed into (n_node, 2), each node's in the order of a loop over
+        vertices, then elements."""
+        if self._node_items is None:
+            flat, item = torch.sort(self.elem_nodes_t.T.reshape(-1), stable=True)
+            start = torch.searchsorted(flat, torch.arange(self._n_node + 1, device=self.device))
+            self._node_items = (start, item)
+        start, item = self._node_items
+        out = torch.zeros((n_node, 2), dtype=torch.float64, device=self.device)
+        capi.check(self.lib.nzb_node_sums(gvert.data_ptr(), start.data_ptr(), item.data_ptr(), self._n_node, item.numel(),
+                                          out.data_ptr(), self.stream), "nzb_node_sums")
+        return out
 
     # -- kernels -------------------------------------------------------------------
     def residual(self, U_soa, X=None, p_back=None):
         """(R, wave) at (U, X, p_back); R unfolded, SoA."""
-        mesh = self.mesh_at(X)
-        ph = self.physics_at(p_back)
+        mesh, pb = self._at(X, p_back)
+        ph = self.physics_at(pb)
         out = torch.empty_like(U_soa)
         wave = torch.empty(self.E, dtype=torch.float64, device=self.device)
         capi.check(self.lib.nzb_residual(C.byref(mesh.c), C.byref(ph), 0, U_soa.data_ptr(), out.data_ptr(),
                                          wave.data_ptr(), self.stream), "nzb_residual")
         return out, wave
 
-    def _vjp(self, mode, U_soa, lam_soa, seed_soa=None, out=None, p_back=None, X=None):
+    def _vjp(self, mode, U_soa, lam_soa, seed_soa=None, out=None, p_back=None, X=None, mesh=None):
         a = capi.AdjointArgs()
         a.mode = mode
         a.U, a.lam = U_soa.data_ptr(), lam_soa.data_ptr()
@@ -130,8 +169,10 @@ class AdjointModel:
         a.out = out.data_ptr() if out is not None else None
         if mode == capi.ADJ_DEFECT:
             a.norm_partial = self._partial.data_ptr()
+        if mesh is None:
+            mesh, p_back = self._at(X, p_back)
         ph = self.physics_at(p_back)
-        capi.check(self.lib.nzb_vjp(C.byref(self.mesh_at(X).c), C.byref(ph), C.byref(a), self.stream), "nzb_vjp")
+        capi.check(self.lib.nzb_vjp(C.byref(mesh.c), C.byref(ph), C.byref(a), self.stream), "nzb_vjp")
 
     def vjp_state(self, U_soa, lam_soa, p_back=None, X=None):
         """(dR/dU)^T lam, SoA."""
@@ -156,11 +197,15 @@ class AdjointModel:
     def vjp_coords_vertices(self, U_soa, lam_soa, X=None, p_back=None):
         """Per element vertex (2, NV, E) d(lam . R)/dX and per element (E) d(lam . R)/dp_back."""
         X = self.X0 if X is None else X
+        mesh, pb = self._at(X, p_back)
+        return self._coords(U_soa, lam_soa, X, mesh, pb)
+
+    def _coords(self, U_soa, lam_soa, X, mesh, p_back):
         ph = self.physics_at(p_back)
         gvert = torch.empty(2 * self.NV * self.E, dtype=torch.float64, device=self.device)
         gpb = torch.empty(self.E, dtype=torch.float64, device=self.device)
         verts = self.verts(X)
-        capi.check(self.lib.nzb_vjp_coords(C.byref(self.mesh_at(X).c), C.byref(ph), U_soa.data_ptr(),
+        capi.check(self.lib.nzb_vjp_coords(C.byref(mesh.c), C.byref(ph), U_soa.data_ptr(),
                                            lam_soa.data_ptr(), verts.data_ptr(), self.dgs.ctypes.data, gvert.data_ptr(),
                                            gpb.data_ptr(), self.stream), "nzb_vjp_coords")
         return gvert.reshape(2, self.NV, self.E), gpb
@@ -169,18 +214,13 @@ class AdjointModel:
         """((dR/dX)^T lam as an (N_nodes, 2) tensor, (dR/dp_back)^T lam as a float)."""
         X = self.X0 if X is None else X
         gv, gpb = self.vjp_coords_vertices(U_soa, lam_soa, X, p_back)
-        # element vertices -> nodes, summed in a fixed order on the host (E x NV entries)
-        gv = gv.cpu().numpy()
-        g = np.zeros((X.shape[0], 2))
-        np.add.at(g[:, 0], self.elem_nodes.T, gv[0])
-        np.add.at(g[:, 1], self.elem_nodes.T, gv[1])
-        return torch.as_tensor(g, device=X.device), float(np.sum(gpb.cpu().numpy()))
+        return self._node_sums(gv, X.shape[0]).to(X.device), float(gpb.sum().item())
 
 
 class _Residual(torch.autograd.Function):
     @staticmethod
     def forward(ctx, model, U, X, p_back):
-        R, _ = model.residual(U.detach().contiguous(), X.detach(), float(p_back))
+        R, _ = model.residual(U.detach().contiguous(), X.detach(), p_back.detach())
         ctx.model = model
         ctx.save_for_backward(U.detach(), X.detach(), p_back.detach())
         return R
@@ -188,15 +228,18 @@ class _Residual(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gR):
         U, X, pb = ctx.saved_tensors
+        U = U.contiguous()
         m = ctx.model
         gR = gR.contiguous()
         gU = gX = gpb = None
+        mesh, p_back = m._at(X, pb)
         if ctx.needs_input_grad[1]:
-            gU = m.vjp_state(U, gR, float(pb), X)
+            gU = torch.empty_like(U)
+            m._vjp(capi.ADJ_VJP, U, gR, out=gU, p_back=p_back, mesh=mesh)
         if ctx.needs_input_grad[2] or ctx.needs_input_grad[3]:
-            g, gp = m.vjp_coords(U, gR, X, float(pb))
-            gX = g.to(dtype=X.dtype, device=X.device)
-            gpb = torch.tensor(gp, dtype=pb.dtype, device=pb.device)
+            gv, gp = m._coords(U, gR, X, mesh, p_back)
+            gX = m._node_sums(gv, X.shape[0]).to(dtype=X.dtype, device=X.device)
+            gpb = gp.sum().to(dtype=pb.dtype, device=pb.device).reshape(pb.shape)
         return None, gU, gX, gpb
 
 

@@ -307,6 +307,9 @@ SIGNATURES = [
     ("nzb_batch_run", C.c_int, [P, C.c_int, C.c_int, P]),
     ("nzb_batch_destroy", C.c_int, [P]),
     ("nzb_vjp", C.c_int, [C.POINTER(Mesh), C.POINTER(Physics), C.POINTER(AdjointArgs), P]),
+    ("nzb_all_close", C.c_int, [P, P, I64, C.c_double, C.c_double, P, P]),
+    ("nzb_element_vertices", C.c_int, [P, P, I64, C.c_int, P, P]),
+    ("nzb_node_sums", C.c_int, [P, P, P, I64, I64, P, P]),
     ("nzb_vjp_coords", C.c_int, [C.POINTER(Mesh), C.POINTER(Physics), P, P, P, P, P, P, P]),
     ("nzb_local_dt", C.c_int, [C.POINTER(Mesh), P, C.c_double, P, P]),
     ("nzb_adjoint_create", C.c_int, [C.c_int, C.POINTER(Mesh), C.POINTER(Physics), C.POINTER(AdjointBuffers), P,

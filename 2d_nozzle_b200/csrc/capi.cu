@@ -526,6 +526,45 @@ __global__ void __launch_bounds__(CHECK_THREADS) k_adjoint_check(nzb_adjoint_mar
   if (st == 0) atomicAdd(am.n_running, 1);
 }
 
+// ---- node coordinates of the differentiable residual ---------------------------------
+// flag = 1 where some |a - b| > atol + rtol |b| (or is a NaN), as allclose; the caller zeroes it.
+__global__ void __launch_bounds__(NT) k_all_close(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
+                                                  double rtol, double atol, double* __restrict__ flag) {
+  const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
+  const bool far = t < n && !(fabs(a[t] - b[t]) <= atol + rtol * fabs(b[t]));
+  if (__syncthreads_or(far) && threadIdx.x == 0) *flag = 1.0;
+}
+
+// (2 NV, E) vertex coordinates of every element from the (n_node, 2) node coordinates.
+__global__ void __launch_bounds__(NT) k_element_vertices(const double* __restrict__ X, const int64_t* __restrict__ elem_nodes,
+                                                         int64_t E, int nv, double* __restrict__ verts) {
+  const int64_t e = (int64_t)blockIdx.x * NT + threadIdx.x;
+  if (e >= E) return;
+  for (int v = 0; v < nv; ++v) {
+    const int64_t n = elem_nodes[e * nv + v];
+    verts[v * E + e] = X[2 * n];
+    verts[(nv + v) * E + e] = X[2 * n + 1];
+  }
+}
+
+// Element-vertex values (2, NV E) summed into nodes (n_node, 2): node n's items are item[start[n] ..
+// start[n + 1]), in increasing order, so the sum's order is fixed -- the order of a loop over vertices,
+// then elements.  One thread per node; a node has at most a handful of items.
+__global__ void __launch_bounds__(NT) k_node_sums(const double* __restrict__ gvert, const int64_t* __restrict__ start,
+                                                  const int64_t* __restrict__ item, int64_t n_node, int64_t n_item,
+                                                  double* __restrict__ out) {
+  const int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x;
+  if (n >= n_node) return;
+  double x = 0.0, y = 0.0;
+  for (int64_t k = start[n]; k < start[n + 1]; ++k) {
+    const int64_t i = item[k];
+    x += gvert[i];
+    y += gvert[n_item + i];
+  }
+  out[2 * n] = x;
+  out[2 * n + 1] = y;
+}
+
 struct AdjBatch {
   std::vector<nzb_mesh> mesh;
   std::vector<nzb_physics> phys;
@@ -1160,6 +1199,25 @@ int nzb_vjp_coords(const nzb_mesh* mesh, const nzb_physics* phys, const double* 
   for (int f = 0; f < 4; ++f)
     for (int v = 0; v < 4; ++v) w.dgs[f][v] = dgs[4 * f + v];
   return dispatch_vjp_coords(*mesh, *phys, w, (cudaStream_t)stream);
+}
+
+int nzb_all_close(const double* a, const double* b, int64_t n, double rtol, double atol, double* flag, void* stream) {
+  if (!a || !b || !flag || n <= 0) return fail("all_close: bad arguments");
+  k_all_close<<<(unsigned)blocks_for(n), NT, 0, (cudaStream_t)stream>>>(a, b, n, rtol, atol, flag);
+  return launch_check("all_close launch");
+}
+
+int nzb_element_vertices(const double* X, const int64_t* elem_nodes, int64_t E, int nv, double* verts, void* stream) {
+  if (!X || !elem_nodes || !verts || E <= 0 || nv <= 0) return fail("element_vertices: bad arguments");
+  k_element_vertices<<<(unsigned)blocks_for(E), NT, 0, (cudaStream_t)stream>>>(X, elem_nodes, E, nv, verts);
+  return launch_check("element_vertices launch");
+}
+
+int nzb_node_sums(const double* gvert, const int64_t* start, const int64_t* item, int64_t n_node, int64_t n_item,
+                  double* out, void* stream) {
+  if (!gvert || !start || !item || !out || n_node <= 0 || n_item <= 0) return fail("node_sums: bad arguments");
+  k_node_sums<<<(unsigned)blocks_for(n_node), NT, 0, (cudaStream_t)stream>>>(gvert, start, item, n_node, n_item, out);
+  return launch_check("node_sums launch");
 }
 
 int nzb_local_dt(const nzb_mesh* mesh, const double* wave, double coefficient, double* dt, void* stream) {

@@ -363,6 +363,16 @@ int nzb_vjp(const nzb_mesh* mesh, const nzb_physics* phys, const nzb_adjoint_arg
 int nzb_vjp_coords(const nzb_mesh* mesh, const nzb_physics* phys, const double* U, const double* lam,
                    const double* verts, const double* dgs, double* gvert, double* gpb, void* stream);
 
+/* Helpers of the differentiable residual's coordinate product.  nzb_all_close sets *flag = 1 where some
+ * |a - b| > atol + rtol |b| (the caller zeroes it).  nzb_element_vertices writes the (2 NV, E) vertex
+ * coordinates nzb_vjp_coords takes from (n_node, 2) coordinates and (E, NV) vertex ids (all in range).
+ * nzb_node_sums sums (2, NV E) element-vertex values into (n_node, 2): node n's items, item[start[n]] to
+ * item[start[n + 1] - 1], are positions v E + e in increasing order, which fixes the order of each sum. */
+int nzb_all_close(const double* a, const double* b, int64_t n, double rtol, double atol, double* flag, void* stream);
+int nzb_element_vertices(const double* X, const int64_t* elem_nodes, int64_t E, int nv, double* verts, void* stream);
+int nzb_node_sums(const double* gvert, const int64_t* start, const int64_t* item, int64_t n_node, int64_t n_item,
+                  double* out, void* stream);
+
 /* dt_e = coefficient * 2 A_e / max(wave_e, 1e-10): local_time_step
  * (src/timestepping/step.py:171-183). */
 int nzb_local_dt(const nzb_mesh* mesh, const double* wave, double coefficient, double* dt, void* stream);
