@@ -59,6 +59,7 @@ struct AdjWork {
   double* norm_partial;  // defect: per-block sum of squares (nullable)
   double* elem_norm;     // defect: per-element sum of squares (nullable)
   const double* jac;     // the face points' flux Jacobians (k_tile_jac), or null: differentiated here
+  bool chained;          // this launch follows a kernel of the same run (tile.cuh)
 };
 
 struct CoordWork {

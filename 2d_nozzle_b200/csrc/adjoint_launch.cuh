@@ -15,10 +15,12 @@ namespace nzb {
 namespace {
 
 template <int K, int P, bool AFF, bool JAC>
-void launch_tile_vjp(const nzb_mesh& m, const nzb_physics& ph, const AdjWork& w, int64_t blocks, cudaStream_t st) {
+cudaError_t launch_tile_vjp(const nzb_mesh& m, const nzb_physics& ph, const AdjWork& w, int64_t blocks, cudaStream_t st) {
   using L = TileVjpSmem<K, P, AFF, JAC>;
   constexpr int64_t most = 148 * L::MINB;  // persistent CTAs: the resident ones of a B200
-  k_tile_vjp<K, P, AFF, JAC><<<(unsigned)(blocks < most ? blocks : most), TILE_WARPS * 32, L::BYTES, st>>>(m, ph, w);
+  // chained only within one wave: past it the dependents' waiting CTAs would hold slots
+  return launch_chained(w.chained && blocks <= most, k_tile_vjp<K, P, AFF, JAC>, (unsigned)(blocks < most ? blocks : most), TILE_WARPS * 32, L::BYTES, st,
+                        m, ph, w);
 }
 
 template <int K, int P, bool AFF>
@@ -27,11 +29,8 @@ cudaError_t launch_vjp(const nzb_mesh& m, const nzb_physics& ph, const AdjWork& 
     if (m.vjp_split == TILE_LANES) {
       const int64_t blocks = m.vjp_blocks ? m.n_vjp_blocks : (m.n_elem + TILE_EB - 1) / TILE_EB;
       if (blocks == 0) return cudaSuccess;
-      if (w.jac)
-        launch_tile_vjp<K, P, AFF, true>(m, ph, w, blocks, st);
-      else
-        launch_tile_vjp<K, P, AFF, false>(m, ph, w, blocks, st);
-      return cudaGetLastError();
+      return w.jac ? launch_tile_vjp<K, P, AFF, true>(m, ph, w, blocks, st)
+                   : launch_tile_vjp<K, P, AFF, false>(m, ph, w, blocks, st);
     }
   }
   const int64_t nb = m.vjp_blocks ? m.n_vjp_blocks : (m.n_elem + Launch<K, P>::NT - 1) / Launch<K, P>::NT;

@@ -92,6 +92,8 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 2)
   const int lane = threadIdx.x & 31, l = lane & 3;
   const int64_t E = m.n_elem, plane = S::NP * E;
   const double* fr = (K == 0 ? g_tile_tri : g_tile_quad) + tile_offset<K>(P) + lane;
+  chain_release();
+  chain_wait();
   const int64_t blk = listed_block(m.vjp_blocks, E, TILE_EB);
   const int64_t tile = blk * TILE_WARPS + (threadIdx.x >> 5), e = tile * TILE_E + (lane >> 2);
   int inst = -1, ccode = 0, cnb = -1, ck = -1;
@@ -212,13 +214,10 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
   // one tile ahead, as in the forward kernel
   int64_t blk = 0;
   int inst = -1, ccode = 0, cnb = -1, ck = -1;
-  auto fetch = [&](int64_t at, double* buf) {
+  auto fetch = [&](int64_t at, double* buf, bool first_tile = false) {
     blk = listed_block(m.vjp_blocks, E, TILE_EB, at);
     const int64_t e0 = blk * TILE_EB + warp * TILE_E, e = e0 + (lane >> 2);
-    copy_rows(buf, w.U, S::NP * 4, E, e0, E);
-    copy_rows(buf + L::STATE, w.lam, S::NP * 4, E, e0, E);
     copy_rows(buf + 2 * L::STATE, m.geo, TileGeo<K, AFF>::ROWS, E, e0, E);
-    copy_commit();
     inst = ccode = 0;
     cnb = ck = -1;
     if (e < E) {
@@ -229,6 +228,10 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
         ck = __ldg(m.face_edge + l * E + e);
       }
     }
+    if (first_tile) chain_wait();  // the states, below, are the previous kernel's
+    copy_rows(buf, w.U, S::NP * 4, E, e0, E);
+    copy_rows(buf + L::STATE, w.lam, S::NP * 4, E, e0, E);
+    copy_commit();
     // what is read straight from global memory later: the Jacobian lines and the epilogue's rows
     if (e0 < E) {
       if constexpr (JAC) {
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
       }
     }
   };
-  fetch(blockIdx.x, wbuf);
+  fetch(blockIdx.x, wbuf, true);
   __syncthreads();  // the staged fragments
 
   int cur = 0;
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
     const int64_t off = l * E + e;  // node 4c + l, component s: off + 4cE + s plane
     cur ^= 1;
     const bool more = b + gridDim.x < blocks;
+    if (!more) chain_release();
     double dsq = 0.0;
     copy_wait<0>();
     if (more) fetch(b + gridDim.x, wbuf + cur * L::BUF);

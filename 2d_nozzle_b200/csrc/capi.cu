@@ -225,8 +225,9 @@ struct Solver {
   std::map<int, cudaGraphExec_t> graphs;
 };
 
-static int enqueue_step(const Solver& s, cudaStream_t st) {
+static int enqueue_step(const Solver& s, bool first, cudaStream_t st) {
   Work w{};
+  w.chained = !first;
   w.op = OP_STAGE;
   w.dt = s.buf.dt;
   w.counters = s.buf.counters;
@@ -247,6 +248,7 @@ static int enqueue_step(const Solver& s, cudaStream_t st) {
                       "euler copy-back");
   }
   w.norm_partial = nullptr;
+  w.chained = true;
   // stage 2: S1 = limit(3/4 S0 + 1/4 (S2 + dt F(S2)))
   w.V = s.buf.S2;
   w.U0 = s.buf.S0;
@@ -274,7 +276,7 @@ static int graph_for(Solver& s, int n, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   if (cuda_check(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal), "begin capture")) return -1;
   int rc = 0;
-  for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_step(s, s.stream);
+  for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_step(s, i == 0, s.stream);
   const cudaError_t end = cudaStreamEndCapture(s.stream, &g);
   if (rc) {
     if (g) cudaGraphDestroy(g);
@@ -393,13 +395,14 @@ struct Batch {
   std::map<int, cudaGraphExec_t> graphs;  // key: 2 * n + first
 };
 
-static int enqueue_bucket_step(const Batch& B, size_t b, cudaStream_t st) {
+static int enqueue_bucket_step(const Batch& B, size_t b, bool first, cudaStream_t st) {
   {
     const nzb_mesh& m = B.mesh[b];
     if (m.fwd_blocks && m.n_fwd_blocks == 0) return 0;  // every instance of the bucket has retired
     const nzb_buffers& bf = B.buf[b];
     const bool ssp = m.order > 0;
     Work w{};
+    w.chained = !first;
     w.op = OP_STAGE;
     w.dt = bf.dt;
     w.dt_factor = B.factor[b];
@@ -417,6 +420,7 @@ static int enqueue_bucket_step(const Batch& B, size_t b, cudaStream_t st) {
       return launch_check("masked copy");
     }
     w.elem_norm = nullptr;
+    w.chained = true;
     w.V = bf.S2;
     w.U0 = bf.S0;
     w.out = bf.S1;
@@ -447,7 +451,7 @@ static int batch_graph(Batch& B, int n, int first, cudaGraphExec_t* out) {
   int rc = cuda_check(cudaEventRecord(B.fork, B.stream), "fork record");
   for (size_t b = 0; b < B.mesh.size() && rc == 0; ++b) {
     rc = cuda_check(cudaStreamWaitEvent(B.bstream[b], B.fork, 0), "fork wait");
-    for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_bucket_step(B, b, B.bstream[b]);
+    for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_bucket_step(B, b, i == 0, B.bstream[b]);
     if (rc == 0) rc = cuda_check(cudaEventRecord(B.bdone[b], B.bstream[b]), "join record");
     if (rc == 0) rc = cuda_check(cudaStreamWaitEvent(B.stream, B.bdone[b], 0), "join wait");
   }
@@ -582,7 +586,7 @@ struct AdjBatch {
   std::map<int, cudaGraphExec_t> graphs;  // key: steps per chunk
 };
 
-static int enqueue_adjoint_step(const AdjBatch& A, size_t b, cudaStream_t st) {
+static int enqueue_adjoint_step(const AdjBatch& A, size_t b, bool first, cudaStream_t st) {
   const nzb_adjoint_buffers& bf = A.buf[b];
   AdjWork w{};
   w.mode = ADJ_RK4;
@@ -598,6 +602,7 @@ static int enqueue_adjoint_step(const AdjBatch& A, size_t b, cudaStream_t st) {
   const double* in[4] = {bf.lam, bf.Y1, bf.Y2, bf.Y1};
   double* outp[4] = {bf.Y1, bf.Y2, bf.Y1, nullptr};
   for (int k = 0; k < 4; ++k) {
+    w.chained = !(first && k == 0);
     w.stage = k;
     w.lam = in[k];
     w.out = outp[k];
@@ -606,7 +611,7 @@ static int enqueue_adjoint_step(const AdjBatch& A, size_t b, cudaStream_t st) {
   return 0;
 }
 
-static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, bool jac, cudaStream_t st) {
+static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, int n, cudaStream_t st) {
   const nzb_adjoint_buffers& bf = A.buf[b];
   AdjWork w{};
   w.mode = ADJ_DEFECT;
@@ -614,7 +619,8 @@ static int enqueue_adjoint_defect(const AdjBatch& A, size_t b, bool jac, cudaStr
   w.seed = bf.seed;
   w.lam = bf.lam;
   w.elem_norm = A.am.elem_norm + A.offset[b];
-  w.jac = jac ? A.jac[b] : nullptr;
+  w.jac = n > 0 ? A.jac[b] : nullptr;
+  w.chained = n > 0;
   return dispatch_vjp(A.mesh[b], A.phys[b], w, st);
 }
 
@@ -636,8 +642,8 @@ static int adjoint_graph(AdjBatch& A, int n, cudaGraphExec_t* out) {
                                         : vjp_jac_launch_quad(m, A.phys[b], A.buf[b].U, A.jac[b], A.bstream[b]),
                       "face Jacobian launch");
     }
-    for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_adjoint_step(A, b, A.bstream[b]);
-    if (rc == 0) rc = enqueue_adjoint_defect(A, b, n > 0, A.bstream[b]);
+    for (int i = 0; i < n && rc == 0; ++i) rc = enqueue_adjoint_step(A, b, i == 0, A.bstream[b]);
+    if (rc == 0) rc = enqueue_adjoint_defect(A, b, n, A.bstream[b]);
     if (rc == 0) rc = cuda_check(cudaEventRecord(A.bdone[b], A.bstream[b]), "join record");
     if (rc == 0) rc = cuda_check(cudaStreamWaitEvent(A.stream, A.bdone[b], 0), "join wait");
   }

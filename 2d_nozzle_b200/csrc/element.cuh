@@ -48,6 +48,7 @@ struct Work {
   uint8_t* flags;
   double dt_factor, a, b;
   int stage;
+  bool chained;  // this launch follows a kernel of the same run (tile.cuh)
 };
 
 template <int K, int P>

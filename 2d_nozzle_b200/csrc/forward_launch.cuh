@@ -39,10 +39,12 @@ cudaError_t superbee_passes(const nzb_mesh& m, const nzb_physics& ph, const doub
 // Persistent CTAs, as many as the GPU holds at once: the tables are staged once per
 // CTA, and a warp prefetches its next tile while it works on one.
 template <int K, int P, bool AFF, bool LIM>
-void launch_tile(const nzb_mesh& m, const nzb_physics& ph, const Work& w, int64_t blocks, cudaStream_t st) {
+cudaError_t launch_tile(const nzb_mesh& m, const nzb_physics& ph, const Work& w, int64_t blocks, cudaStream_t st) {
   using L = TileSmem<K, P, AFF, LIM>;
   constexpr int64_t most = 148 * L::MINB;
-  k_tile<K, P, AFF, LIM><<<(unsigned)(blocks < most ? blocks : most), TILE_WARPS * 32, L::BYTES, st>>>(m, ph, w);
+  // chained only within one wave: past it the dependents' waiting CTAs would hold slots
+  return launch_chained(w.chained && blocks <= most, k_tile<K, P, AFF, LIM>, (unsigned)(blocks < most ? blocks : most), TILE_WARPS * 32, L::BYTES, st, m,
+                        ph, w);
 }
 
 inline cudaError_t first_error(std::initializer_list<cudaError_t> all) {
@@ -71,12 +73,11 @@ cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cuda
   if constexpr (P > 0) {
     if (m.split == TILE_LANES) {
       const int64_t blocks = m.fwd_blocks ? m.n_fwd_blocks : (m.n_elem + TILE_EB - 1) / TILE_EB;
-      if (blocks == 0)
-        ;  // an empty block list: nothing marches
-      else if (lim)
-        launch_tile<K, P, AFF, true>(m, ph, w, blocks, st);
-      else
-        launch_tile<K, P, AFF, false>(m, ph, w, blocks, st);
+      if (blocks > 0) {  // an empty block list: nothing marches
+        const cudaError_t e = lim ? launch_tile<K, P, AFF, true>(m, ph, w, blocks, st)
+                                  : launch_tile<K, P, AFF, false>(m, ph, w, blocks, st);
+        if (e != cudaSuccess) return e;
+      }
       done = true;
     }
   }

@@ -24,8 +24,7 @@ cudaError_t launch_element(const nzb_gen_mesh& m, const nzb_physics& ph, const G
   int bytes = 0;
   const cudaError_t e = warp_smem(k_gen_element<MT>, m, &bytes);
   if (e != cudaSuccess) return e;
-  k_gen_element<MT><<<warp_blocks(m.n_elem), GEN_WARPS * 32, bytes, st>>>(m, ph, w);
-  return cudaGetLastError();
+  return launch_chained(w.chained, k_gen_element<MT>, warp_blocks(m.n_elem), GEN_WARPS * 32, bytes, st, m, ph, w);
 }
 
 cudaError_t element_pass(const nzb_gen_mesh& m, const nzb_physics& ph, const GenWork& w, cudaStream_t st) {
@@ -40,18 +39,18 @@ cudaError_t element_pass(const nzb_gen_mesh& m, const nzb_physics& ph, const Gen
 }
 
 cudaError_t edge_pass(const nzb_gen_mesh& m, const nzb_physics& ph, const double* U, double* fw, double* smax,
-                      cudaStream_t st) {
-  k_gen_edge<<<blocks(8 * (m.n_int + m.n_bnd)), 128, 0, st>>>(m, ph, U, fw, smax);
-  return cudaGetLastError();
+                      bool chained, cudaStream_t st) {
+  return launch_chained(chained, k_gen_edge, blocks(8 * (m.n_int + m.n_bnd)), 128, 0, st, m, ph, U, fw, smax);
 }
 
 }  // namespace
 
 cudaError_t gen_rate_launch(const nzb_gen_mesh& m, const nzb_physics& ph, int unfolded, const double* U, double* out,
                             double* wave, double* fw, double* smax, cudaStream_t st) {
-  const cudaError_t e = edge_pass(m, ph, U, fw, smax, st);
+  const cudaError_t e = edge_pass(m, ph, U, fw, smax, false, st);
   if (e != cudaSuccess) return e;
   GenWork w{};
+  w.chained = true;
   w.op = unfolded ? GEN_RESIDUAL : GEN_RATE;
   w.V = U;
   w.out = out;
@@ -75,10 +74,13 @@ cudaError_t gen_limit_launch(const nzb_gen_mesh& m, const nzb_physics& ph, doubl
 // limiter; the Superbee limiter's passes follow it where that is the limiter.
 cudaError_t gen_run_launch(const nzb_gen_mesh& m, const nzb_physics& ph, const nzb_gen_run_args& r, int n_steps,
                            cudaStream_t st) {
+  bool first = true;
   auto stage = [&](int k, const double* V, const double* U0, double* out, double a, double b) -> cudaError_t {
-    cudaError_t e = edge_pass(m, ph, V, r.fw, r.smax, st);
+    cudaError_t e = edge_pass(m, ph, V, r.fw, r.smax, !first, st);
     if (e != cudaSuccess) return e;
+    first = false;
     GenWork w{};
+    w.chained = true;
     w.op = GEN_STAGE;
     w.stage = k;
     w.limit = ph.limiter == 1;

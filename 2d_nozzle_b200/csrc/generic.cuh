@@ -55,6 +55,7 @@ enum { GEN_RESIDUAL = 0, GEN_RATE = 1, GEN_STAGE = 2, GEN_LIMIT = 3 };
 
 struct GenWork {
   int op, stage, limit;    // limit: the positivity limiter ends the stage
+  bool chained;            // this launch follows a kernel of the same call (tile.cuh)
   const double* V;         // state the rate is evaluated at (the limiter's state)
   const double* U0;        // step start state (a != 0)
   double* out;
@@ -99,9 +100,11 @@ __device__ __forceinline__ double warp_min(double v) {
 
 __global__ void __launch_bounds__(128) k_gen_edge(const nzb_gen_mesh m, const nzb_physics ph, const double* __restrict__ U,
                                                   double* __restrict__ fw, double* __restrict__ smax) {
+  chain_release();
   const int64_t n_edge = m.n_int + m.n_bnd;
   const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   double best = 0.0;
+  chain_wait();
   if (k < n_edge) {
     const int np = m.np, nqf = m.nqf, nf = m.nface;
     const bool interior = k < m.n_int;
@@ -274,6 +277,8 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_element(const nzb_gen_me
   double* const sp = su + 4 * np;
   const int64_t e = (int64_t)blockIdx.x * GEN_WARPS + (threadIdx.x >> 5);
   int scaled = 0, repaired = 0;
+  chain_release();
+  chain_wait();
   if (e < m.n_elem) {
     const int64_t base = e * np * 4;
     for (int k = lane; k < np * 4; k += 32) su[k] = w.V[base + k];

@@ -333,6 +333,35 @@ __device__ __forceinline__ double quad_min(double v) {
   return o < v ? o : v;
 }
 
+// ---- launches that overlap their predecessor's tail --------------------------------
+// A march is a chain of short dependent kernels.  Each but the first of a run is
+// launched as a programmatic dependent of the one before it: its CTAs may start
+// while that one drains (once all its CTAs have called chain_release), stage their
+// tables and read the mesh's own arrays, and wait in chain_wait() before they touch
+// anything a kernel of the chain writes.  chain_wait returns when the earlier kernel
+// has completed and its writes are visible, and every kernel of a chain calls it, so
+// that holds for all earlier ones; without such a launch both are no-ops.  The mesh's
+// arrays are read before the wait, so a launch is chained only where the call itself
+// put a kernel of the chain in front of it -- never right after work of the caller's
+// (which may have written them, as nzb_geometry does).
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned blocks, unsigned threads, int smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- asynchronous copies: a tile's rows ------------------------------------------
 // Copy `rows` rows of eight consecutive doubles (row r at src + r * stride + e0) into
 // dst[8 r + 0..7], elements past E as zeros.  Eight bytes per lane: rows start at any

@@ -349,12 +349,10 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
   // instance and (face l in lane l) its connectivity.
   int64_t blk = 0;
   int inst = -1, ccode = 0, cnb = -1, ck = -1;
-  auto fetch = [&](int64_t at, double* buf) {
+  auto fetch = [&](int64_t at, double* buf, bool first_tile = false) {
     blk = listed_block(m.fwd_blocks, E, TILE_EB, at);
     const int64_t e0 = blk * TILE_EB + warp * TILE_E, e = e0 + (lane >> 2);
-    copy_rows(buf, w.V, S::NP * 4, E, e0, E);
     copy_rows(buf + L::STATE, m.geo, TileGeo<K, AFF>::ROWS, E, e0, E);
-    copy_commit();
     inst = ccode = 0;
     cnb = ck = -1;
     if (e < E) {
@@ -365,8 +363,11 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
         ck = __ldg(m.face_edge + l * E + e);
       }
     }
+    if (first_tile) chain_wait();  // the states, below, are the previous kernel's
+    copy_rows(buf, w.V, S::NP * 4, E, e0, E);
+    copy_commit();
   };
-  fetch(blockIdx.x, wbuf);
+  fetch(blockIdx.x, wbuf, true);
   __syncthreads();  // the staged fragments
 
   int cur = 0;
@@ -380,6 +381,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
     const int64_t off = l * E + e;                // node 4c + l, component s: off + 4cE + s plane
     cur ^= 1;
     const bool more = b + gridDim.x < blocks;
+    if (!more) chain_release();
     double nrm = 0.0;
     int scaled = 0, repaired = 0;
 
