@@ -28,6 +28,7 @@
 // also forms the Jacobians once (163 us, a dual-number product in place 236).
 #pragma once
 #include "adjoint.cuh"
+#include "flux.cuh"
 #include "tile.cuh"
 
 namespace nzb {
@@ -160,7 +161,7 @@ __device__ __forceinline__ bool lean_flux_vjp(const double (&U)[4], double g, co
   const double rho = U[0];
   b[0] = b[1] = b[2] = b[3] = 0.0;
   if (!(rho >= FLOOR)) return false;
-  const double r = 1.0 / rho;
+  const double r = lean_rcp(rho);
   const double u = U[1] * r, v = U[2] * r;
   const double q2 = u * u + v * v;
   const double gm = g - 1.0;
@@ -470,13 +471,13 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
         apply(T::A_MI);
         double scale = 1.0;
         if constexpr (K == 0) {
-          scale = act ? -1.0 / geo.g[4] : 0.0;
+          scale = act ? -lean_rcp(geo.g[4]) : 0.0;
         } else {
 #pragma unroll
           for (int c = 0; c < T::NS; ++c) {
             double x0, x1, x2, x3;
             const double det = geo.at(fr[(T::A_XI + c) * 32], fr[(T::A_ETA + c) * 32], x0, x1, x2, x3);
-            const double z = act && 4 * c + l < S::NP ? -1.0 / (fr[(T::A_WV + c) * 32] * det) : 0.0;
+            const double z = act && 4 * c + l < S::NP ? -lean_rcp(fr[(T::A_WV + c) * 32] * det) : 0.0;
 #pragma unroll
             for (int s = 0; s < 4; ++s) d[c][s] = r[c >> 1][s][c & 1] * z;
           }

@@ -16,6 +16,7 @@
 
 #include "adjoint_dispatch.cuh"
 #include "element.cuh"
+#include "flux.cuh"
 #include "forward_dispatch.cuh"
 #include "nozzle_b200.h"
 #include "tile.cuh"
@@ -528,6 +529,14 @@ __global__ void __launch_bounds__(CHECK_THREADS) k_adjoint_check(nzb_adjoint_mar
   }
   am.status[inst] = st;
   if (st == 0) atomicAdd(am.n_running, 1);
+}
+
+__global__ void __launch_bounds__(NT) k_reciprocals(const double* __restrict__ a, double* __restrict__ rcp,
+                                                    double* __restrict__ root, int64_t n) {
+  const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
+  if (t >= n) return;
+  rcp[t] = lean_rcp(a[t]);
+  root[t] = lean_rsqrt(a[t]);
 }
 
 // ---- node coordinates of the differentiable residual ---------------------------------
@@ -1205,6 +1214,12 @@ int nzb_vjp_coords(const nzb_mesh* mesh, const nzb_physics* phys, const double* 
   for (int f = 0; f < 4; ++f)
     for (int v = 0; v < 4; ++v) w.dgs[f][v] = dgs[4 * f + v];
   return dispatch_vjp_coords(*mesh, *phys, w, (cudaStream_t)stream);
+}
+
+int nzb_reciprocals(const double* a, double* rcp, double* rsqrt, int64_t n, void* stream) {
+  if (!a || !rcp || !rsqrt || n <= 0) return fail("reciprocals: bad arguments");
+  k_reciprocals<<<(unsigned)blocks_for(n), NT, 0, (cudaStream_t)stream>>>(a, rcp, rsqrt, n);
+  return launch_check("reciprocals launch");
 }
 
 int nzb_all_close(const double* a, const double* b, int64_t n, double rtol, double atol, double* flag, void* stream) {

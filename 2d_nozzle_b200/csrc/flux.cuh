@@ -1,23 +1,59 @@
-// flux.cuh -- the interface fluxes of physics.cuh with fewer divisions and square
-// roots, for the tile kernels.
+// flux.cuh -- the interface fluxes of physics.cuh with fewer and shorter divisions
+// and square roots, for the tile and the generic kernels.
 //
 // A division or square root is an iterative sequence of a dozen and more
 // instructions and over 100 cycles of latency (a 1 / x chain measured 135 cycles a
 // step, sqrt 103, against 13 for a multiply-add), and they are most of a flux.  One
 // reciprocal gives both traces' 1 / rho; the Roe weights need only
 // r = sqrt(rho_R / rho_L); a square root whose reciprocal is wanted too, or whose
-// argument is known positive, comes as x rsqrt(x).  HLLC goes from 11 divisions and
+// argument is known positive, comes as x / sqrt(x).  HLLC goes from 11 divisions and
 // roots to 8, Roe from 7 (10 inside the entropy fix) to 4, AUSM+-up from 6 to 4.
 // Together with shorter address arithmetic in the loads, a residual of 480 000 linear
 // triangles went 199 -> 173 us, of 240 000 cubic quadrilaterals 235 -> 195 us (tile
 // kernel before its asynchronous copies).  The values differ from the templates' in the last
 // bits, so the one-thread kernels keep those.
 //
-// Arguments of rsqrt are positive: rho and p are floored at FLOOR (a NaN stays one).
+// Arguments of the roots are positive: rho and p are floored at FLOOR (a NaN stays one).
 #pragma once
 #include "physics.cuh"
 
 namespace nzb {
+
+// 1 / a and 1 / sqrt(a) for normal, finite a (a > 0 for the root): the hardware's
+// approximation (rcp / rsqrt.approx.ftz.f64, about 20 bits) and one third-order
+// Householder step -- with e = 1 - a x,  x (1 + e + e^2), and with e = 1 - a y^2,
+// y (1 + e / 2 + 3 e^2 / 8) -- whose remainder, of order e^3 = 2^-60, is below the
+// rounding.  No range checks and no branch, unlike the division and root they
+// replace: three and four multiply-adds (nzb_reciprocals exposes them to the tests).
+// Over 4 x 10^6 arguments per decade, 1e-30 to 1e30, the reciprocal is at most one
+// unit in the last place from the division's, the root's relative error at most
+// 1.26 x 2^-53.  A stage of 480 000 cubic triangles went 380 -> 332 us with them, of
+// 240 000 cubic quadrilaterals 291 -> 260, the 72-member sweep's step 547 -> 493.  An argument of zero, a denormal or an infinity gives a NaN; the floors
+// and guards of the callers keep them above 1e-20, and a NaN stays one.
+__device__ __forceinline__ double lean_rcp(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-a, x, 1.0);
+  return fma(x, fma(e, e, e), x);
+}
+__device__ __forceinline__ double lean_rsqrt(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-(a * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// primitives(U, g) of physics.cuh with lean_rcp.
+__device__ __forceinline__ Prim lean_primitives(const double* U, double g) {
+  Prim s;
+  s.rho = floor_at(U[0], FLOOR);
+  s.inv = lean_rcp(s.rho);
+  s.vx = U[1] * s.inv;
+  s.vy = U[2] * s.inv;
+  s.p = floor_at((g - 1.0) * (U[3] - 0.5 * s.rho * (s.vx * s.vx + s.vy * s.vy)), FLOOR);
+  s.H = (U[3] + s.p) * s.inv;
+  return s;
+}
 
 struct PrimPair {
   Prim L, R;
@@ -27,7 +63,7 @@ __device__ __forceinline__ PrimPair primitive_pair(const double* UL, const doubl
   PrimPair s;
   s.L.rho = floor_at(UL[0], FLOOR);
   s.R.rho = floor_at(UR[0], FLOOR);
-  const double t = 1.0 / (s.L.rho * s.R.rho);
+  const double t = lean_rcp(s.L.rho * s.R.rho);
   s.L.inv = t * s.R.rho;
   s.R.inv = t * s.L.rho;
 #pragma unroll
@@ -50,20 +86,20 @@ __device__ __forceinline__ double lean_roe_flux(const double* UL, const double* 
   normal_flux(L, nx, ny, FL);
   normal_flux(R, nx, ny, FR);
   const double r2 = R.rho * L.inv;
-  const double r = r2 * rsqrt(r2);
-  const double iden = 1.0 / (1.0 + r);
+  const double r = r2 * lean_rsqrt(r2);
+  const double iden = lean_rcp(1.0 + r);
   const double vx = (L.vx + r * R.vx) * iden;
   const double vy = (L.vy + r * R.vy) * iden;
   const double H = (L.H + r * R.H) * iden;
   const double q2 = vx * vx + vy * vy;
   const double c2 = floor_at((g - 1.0) * (H - 0.5 * q2), FLOOR);
-  const double ic = rsqrt(c2), c = c2 * ic;
+  const double ic = lean_rsqrt(c2), c = c2 * ic;
   const double vn = vx * nx + vy * ny;
   double l1 = fabs(vn + c), l2 = fabs(vn - c), l3 = fabs(vn);
   const double smax = l1 < l2 ? l2 : l1;
   const double eps = efix * c;
   if (l1 < eps || l2 < eps || l3 < eps) {
-    const double h = 0.5 / eps, e2 = eps * eps;
+    const double h = 0.5 * lean_rcp(eps), e2 = eps * eps;
     if (l1 < eps) l1 = (l1 * l1 + e2) * h;
     if (l2 < eps) l2 = (l2 * l2 + e2) * h;
     if (l3 < eps) l3 = (l3 * l3 + e2) * h;
@@ -88,16 +124,16 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
   const double aL2 = floor_at(g * L.p * L.inv, FLOOR), aR2 = floor_at(g * R.p * R.inv, FLOOR);
-  const double aL = aL2 * rsqrt(aL2), aR = aR2 * rsqrt(aR2);
+  const double aL = aL2 * lean_rsqrt(aL2), aR = aR2 * lean_rsqrt(aR2);
   const double r2 = R.rho * L.inv;
-  const double r = r2 * rsqrt(r2);
-  const double iden = 1.0 / (1.0 + r);
+  const double r = r2 * lean_rsqrt(r2);
+  const double iden = lean_rcp(1.0 + r);
   const double vx = (L.vx + r * R.vx) * iden;
   const double vy = (L.vy + r * R.vy) * iden;
   const double H = (L.H + r * R.H) * iden;
   const double vt = vx * nx + vy * ny;
   const double at2 = floor_at((g - 1.0) * (H - 0.5 * (vx * vx + vy * vy)), FLOOR);
-  const double at = at2 * rsqrt(at2);
+  const double at = at2 * lean_rsqrt(at2);
   double SL = fmin(vnL - aL, vt - at);
   double SR = fmax(vnR + aR, vt + at);
   if (low_mach > 0.0) {
@@ -110,7 +146,7 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
   const double smax = fmax(fabs(SL), fabs(SR));
   const double mL = L.rho * (SL - vnL), mR = R.rho * (SR - vnR);
   const double dm = fabs(mR - mL) > FLOOR ? mR - mL : FLOOR;
-  const double SM = (vnR * mR - vnL * mL + L.p - R.p) / dm;
+  const double SM = (vnR * mR - vnL * mL + L.p - R.p) * lean_rcp(dm);
   // the side the face lies on: left of SL or of the contact, the left one; its star
   // state applies between SL and SR
   const bool left = SL >= 0.0 || (!(SR <= 0.0) && SM >= 0.0);
@@ -125,7 +161,7 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
   if (star) {
     // U* - U with one reciprocal for 1 / (S - SM) and 1 / (rho (S - vn))
     const double a = guard(S - SM), b = guard(m);
-    const double t = 1.0 / (a * b);
+    const double t = lean_rcp(a * b);
     const double rs = m * (t * b);  // rho (S - vn) / (S - SM)
     const double dv = SM - vn;
     const double Es = E * (left ? L.inv : R.inv) + dv * (SM + p * (t * a));
@@ -145,9 +181,9 @@ __device__ __forceinline__ double lean_ausm_up_flux(const double* UL, const doub
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
   const double aL2 = g * L.p * L.inv, aR2 = g * R.p * R.inv;
-  const double aL = aL2 * rsqrt(aL2), aR = aR2 * rsqrt(aR2);
+  const double aL = aL2 * lean_rsqrt(aL2), aR = aR2 * lean_rsqrt(aR2);
   const double ah = 0.5 * (aL + aR), rh = 0.5 * (L.rho + R.rho);
-  const double t = 1.0 / (ah * rh), iah = t * rh;
+  const double t = lean_rcp(ah * rh), iah = t * rh;
   const double mL = vnL * iah, mR = vnR * iah;
   const double mb2 = 0.5 * (mL * mL + mR * mR);
   const double pL2 = 0.25 * ((mL + 1.0) * (mL + 1.0)), mL2 = -0.25 * ((mL - 1.0) * (mL - 1.0));

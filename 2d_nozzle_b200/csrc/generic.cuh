@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_element(const nzb_gen_me
 #pragma unroll
           for (int s = 0; s < 4; ++s) u[s] = fma(b, su[i * 4 + s], u[s]);
         }
-        const Prim pr = primitives_fast(u, g);
+        const Prim pr = lean_primitives(u, g);
         double* F = sp + q * 8;
         F[0] = pr.rho * pr.vx;
         F[1] = pr.rho * pr.vx * pr.vx + pr.p;

@@ -83,7 +83,7 @@ __device__ __forceinline__ void tile_limit(double (&u)[Tile<K, P>::NS][4], const
 #pragma unroll
       for (int t = 0; t < T::NT; ++t) mma(dm[t], det, fr[(T::MW + v * T::NT + t) * 32]);
     }
-    const double ra = 1.0 / (act ? __ldg(m.area + e) : 1.0);
+    const double ra = lean_rcp(act ? __ldg(m.area + e) : 1.0);
 #pragma unroll
     for (int c = 0; c < T::NS; ++c) mw[c] = dm[c >> 1][c & 1] * ra;
   }
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
             const int v = 2 * vt + j;
             if (T::VS % 2 == 1 && v >= T::VS) continue;
             const double uq[4] = {d[0][j], d[1][j], d[2][j], d[3][j]};
-            const Prim pr = primitives_fast(uq, g);
+            const Prim pr = lean_primitives(uq, g);
             const double F[4] = {pr.rho * pr.vx, pr.rho * pr.vx * pr.vx + pr.p, pr.rho * pr.vx * pr.vy, pr.rho * pr.vx * pr.H};
             const double G[4] = {pr.rho * pr.vy, pr.rho * pr.vx * pr.vy, pr.rho * pr.vy * pr.vy + pr.p, pr.rho * pr.vy * pr.H};
             // triangles: (xi_x F + xi_y G) det, det only for the residual (the rate divides it out
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
 
         // ---- faces
         // triangles' rates: the face term carries -1/det (the rate is -M^-1 R with M = det M_ref)
-        const double fsc = (K == 0 && rate) ? -1.0 / geo.g[4] : 1.0;
+        const double fsc = (K == 0 && rate) ? -lean_rcp(geo.g[4]) : 1.0;
         double wave = 0.0;
 #pragma unroll 1
         for (int fs = 0; fs < T::FS; ++fs) {
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
             double x0, x1, x2, x3;
             const double det = geo.at(fr[(T::XI + c) * 32], fr[(T::ETA + c) * 32], x0, x1, x2, x3);
             const double wd = fr[(T::WV + c) * 32] * det;
-            const double r = act && 4 * c + l < S::NP ? -1.0 / wd : 0.0;
+            const double r = act && 4 * c + l < S::NP ? -lean_rcp(wd) : 0.0;
 #pragma unroll
             for (int s = 0; s < 4; ++s) y[c][s] = acc[c >> 1][s][c & 1] * r;
           }
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
           double dt = scale_t;
           if (!later) {
             const double d = wave < FLOOR ? FLOOR : wave;
-            dt = w.dt_factor * 2.0 * scale_t / d;
+            dt = w.dt_factor * 2.0 * scale_t * lean_rcp(d);
             if (act && l == 0) w.dt[e] = dt;
           }
           // the starting state's rows have landed (the next tile's may still be on their way)

@@ -85,6 +85,25 @@ def test_adjoint_tiles_agree_with_one_thread(cuda, kind, p, nx, nr, monkeypatch)
         assert rel(y.cpu().numpy(), x.cpu().numpy()) < TOL
 
 
+@pytest.mark.parametrize("decade", [-30, -20, -10, -1, 0, 1, 10, 20, 29])
+def test_reciprocals_are_accurate(cuda, decade):
+    """1 / a and 1 / sqrt(a) of the fluxes against the division's and torch's.  The step's remainder is
+    2^-60 relative; two roundings follow it in the reciprocal and three in the root (half a unit each, the
+    first of them scaled by the small correction), and the compared values have half a unit themselves:
+    at most two units in the last place."""
+    import torch
+
+    capi = pkg("capi")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(decade + 100)
+    a = 10.0**decade * (1.0 + 9.0 * torch.rand(200_001, generator=gen, dtype=torch.float64, device="cuda"))
+    r, q = torch.empty_like(a), torch.empty_like(a)
+    capi.check(capi.load().nzb_reciprocals(a.data_ptr(), r.data_ptr(), q.data_ptr(), a.numel(),
+                                           torch.cuda.current_stream().cuda_stream), "nzb_reciprocals")
+    for got, ref in ((r, 1.0 / a), (q, 1.0 / torch.sqrt(a))):
+        assert float(((got - ref).abs() / ref).max()) <= 2 * 2.0**-52
+
+
 def test_a_lone_large_instance_keeps_the_one_thread_kernel():
     """Which buckets the exception to the variant table takes (autotune.bucket_context)."""
     at = pkg("autotune")
