@@ -187,7 +187,7 @@ template <int K, int P, bool AFF, bool JAC>
 struct TileVjpSmem {
   using S = Shape<K, P>;
   using T = Tile<K, P>;
-  static constexpr int FRAGS = (T::COUNT - T::A_PHI) * 32;
+  static constexpr int FRAGS = (T::A_END - T::A_PHI) * 32;
   static constexpr int STATE = S::NP * 4 * TILE_E;
   static constexpr int BUF = 2 * STATE + TileGeo<K, AFF>::ROWS * TILE_E;
   static constexpr int BYTES = (FRAGS + TILE_WARPS * 2 * BUF) * 8;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
   const int lane = threadIdx.x & 31, l = lane & 3, warp = threadIdx.x >> 5;
   const int64_t E = m.n_elem, plane = S::NP * E;
   const double g = ph.gamma;
-  stage_tiles<K, P>(smem, T::A_PHI, T::COUNT - T::A_PHI);
+  stage_tiles<K, P>(smem, T::A_PHI, T::A_END - T::A_PHI);
   const double* fr = smem + lane - T::A_PHI * 32;  // fragment n of this lane is fr[32 n]
   double* const wbuf = smem + L::FRAGS + warp * 2 * L::BUF;
   const int64_t blocks = m.vjp_blocks ? m.n_vjp_blocks : (E + TILE_EB - 1) / TILE_EB;

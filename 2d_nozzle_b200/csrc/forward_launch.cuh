@@ -10,7 +10,8 @@
 //   otherwise      k_element: one thread per element, fluxes from both sides.
 // With the Superbee limiter (limiter 2) the element kernel leaves the stage
 // unlimited and three passes follow (cell means, their maximum -- per
-// instance in a batch -- and the slope limiter with the positivity limiter).
+// instance in a batch -- and the slope limiter with the positivity limiter);
+// the tile kernel forms the means and maxima itself, so one follows it.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -24,6 +25,14 @@ namespace nzb {
 namespace {
 
 template <int K, int P, bool AFF>
+cudaError_t tile_superbee(const nzb_mesh& m, const nzb_physics& ph, const double* V, double* out,
+                          unsigned long long* counters, uint8_t* flags, bool chained, cudaStream_t st) {
+  return launch_chained(chained, k_tile_superbee<K, P, AFF>, (unsigned)((m.n_elem + TILE_EB - 1) / TILE_EB), TILE_WARPS * 32, 0,
+                        st, m, ph, V, out, counters, flags);
+}
+
+// The limiter on a state: averages, their maxima, then the factor, the scaling and the positivity limiter.
+template <int K, int P, bool AFF>
 cudaError_t superbee_passes(const nzb_mesh& m, const nzb_physics& ph, const double* V, double* out,
                             unsigned long long* counters, uint8_t* flags, cudaStream_t st) {
   const unsigned nb = (unsigned)((m.n_elem + 127) / 128);
@@ -32,6 +41,9 @@ cudaError_t superbee_passes(const nzb_mesh& m, const nzb_physics& ph, const doub
     k_lim_scale_inst<<<nb, 128, 0, st>>>(m.lim_means, m.n_elem, m.elem_inst, m.lim_scale);
   else
     k_lim_scale<<<1, 1024, 0, st>>>(m.lim_means, m.n_elem, m.lim_scale);
+  if constexpr (P > 0) {
+    if (m.split == TILE_LANES) return tile_superbee<K, P, AFF>(m, ph, V, out, counters, flags, false, st);
+  }
   k_superbee<K, P, AFF><<<nb, 128, 0, st>>>(m, ph, V, out, counters, flags);
   return cudaGetLastError();
 }
@@ -73,11 +85,19 @@ cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cuda
   if constexpr (P > 0) {
     if (m.split == TILE_LANES) {
       const int64_t blocks = m.fwd_blocks ? m.n_fwd_blocks : (m.n_elem + TILE_EB - 1) / TILE_EB;
+      // Superbee: the stage kernel leaves the averages and, from zero, their maxima; one pass follows
+      Work wt = w;
+      if (sb) {
+        const cudaError_t e = cudaMemsetAsync(m.lim_scale, 0, sizeof(double) * 4 * (m.elem_inst ? m.n_inst : 1), st);
+        if (e != cudaSuccess) return e;
+        wt.chained = false;
+      }
       if (blocks > 0) {  // an empty block list: nothing marches
-        const cudaError_t e = lim ? launch_tile<K, P, AFF, true>(m, ph, w, blocks, st)
-                                  : launch_tile<K, P, AFF, false>(m, ph, w, blocks, st);
+        const cudaError_t e = lim ? launch_tile<K, P, AFF, true>(m, ph, wt, blocks, st)
+                                  : launch_tile<K, P, AFF, false>(m, ph, wt, blocks, st);
         if (e != cudaSuccess) return e;
       }
+      if (sb) return blocks > 0 ? tile_superbee<K, P, AFF>(m, ph, w.out, w.out, w.counters, w.flags, true, st) : cudaSuccess;
       done = true;
     }
   }

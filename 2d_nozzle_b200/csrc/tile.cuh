@@ -85,7 +85,9 @@ struct Tile {
   static constexpr int A_XI = A_WV + (K == 1 ? VS : 0);
   static constexpr int A_ETA = A_XI + (K == 1 ? VS : 0);
   static constexpr int A_WF = A_ETA + (K == 1 ? VS : 0);
-  static constexpr int COUNT = A_WF + 1;
+  static constexpr int A_END = A_WF + 1;
+  static constexpr int FM = A_END;                   // [NS] nodes -> the average over face l, in lane l's even column
+  static constexpr int COUNT = FM + NS;
   // [VS][NT][2 xi, eta] points -> nodes and [FS][NT] face points -> nodes
   static constexpr int vx(int folded, int v, int t, int d) { return (folded ? COMMON_END : 0) + (v * NT + t) * 2 + d; }
   static constexpr int lf(int folded, int fs, int t) { return (folded ? COMMON_END : 0) + VXN + fs * NT + t; }
@@ -264,6 +266,17 @@ std::vector<double> tile_tables(const double* slot) {
     copy(T::A_ETA, T::ETA, T::VS);
   }
   copy(T::A_WF, T::WF, 1);
+  for (int c = 0; c < T::NS; ++c)
+    put(T::FM + c, [&](int k, int j, int l) {
+      const int i = 4 * c + k, e = j == 0 && i < NP && l < NF ? edge_pos(K, P, l, i) : -1;
+      if (e < 0) return 0.0;
+      long double s = 0.0L, w = 0.0L;
+      for (int q = 0; q < NQF; ++q) {
+        s += (long double)wf[q] * pfe[(l * NE + e) * NQF + q];
+        w += wf[q];
+      }
+      return (double)(s / w);
+    });
   return out;
 }
 
