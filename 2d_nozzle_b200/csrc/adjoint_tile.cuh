@@ -24,8 +24,8 @@
 // lambda travel to shared memory.
 //
 // Measured on a B200 (us per RK4 stage, in a march): 2 240 quadratic triangles
-// 23.5 -> 8.5, 143 360 of them (AUSM+-up) 223 -> 140, where a run of steps
-// also forms the Jacobians once (163 us, a dual-number product in place 236).
+// 23.5 -> 5.9, 143 360 of them (AUSM+-up) 223 -> 90, where a run of steps
+// also forms the Jacobians once (163 us; a dual-number product in place takes 217).
 #pragma once
 #include "adjoint.cuh"
 #include "flux.cuh"
@@ -190,9 +190,14 @@ struct TileVjpSmem {
   static constexpr int FRAGS = (T::A_END - T::A_PHI) * 32;
   static constexpr int STATE = S::NP * 4 * TILE_E;
   static constexpr int BUF = 2 * STATE + TileGeo<K, AFF>::ROWS * TILE_E;
-  static constexpr int BYTES = (FRAGS + TILE_WARPS * 2 * BUF) * 8;
-  static constexpr int FIT = (227 * 1024) / (BYTES + 1024);
   static constexpr int WANT = JAC ? 3 : 2;
+  static constexpr int BASE = (FRAGS + TILE_WARPS * 2 * BUF) * 8;
+  static constexpr int EPI_BYTES = TILE_WARPS * 2 * STATE * 8;
+  // the epilogue's dJ/dU and starting lambda travel to shared memory too where that costs no resident block
+  static constexpr bool EPI = (227 * 1024) / (BASE + EPI_BYTES + 1024) >= WANT;
+  static constexpr int WARP = 2 * BUF + (EPI ? 2 * STATE : 0);
+  static constexpr int BYTES = BASE + (EPI ? EPI_BYTES : 0);
+  static constexpr int FIT = (227 * 1024) / (BYTES + 1024);
   static constexpr int MINB = FIT < WANT ? FIT : WANT;
 };
 
@@ -209,7 +214,8 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
   const double g = ph.gamma;
   stage_tiles<K, P>(smem, T::A_PHI, T::A_END - T::A_PHI);
   const double* fr = smem + lane - T::A_PHI * 32;  // fragment n of this lane is fr[32 n]
-  double* const wbuf = smem + L::FRAGS + warp * 2 * L::BUF;
+  double* const wbuf = smem + L::FRAGS + warp * L::WARP;
+  double* const ebuf = wbuf + 2 * L::BUF;  // dJ/dU, then the step's starting lambda (L::EPI)
   const int64_t blocks = m.vjp_blocks ? m.n_vjp_blocks : (E + TILE_EB - 1) / TILE_EB;
 
   // one tile ahead, as in the forward kernel
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
           const int64_t o = r * E + e0;
           prefetch_line(w.seed + o);
           if (w.mode == ADJ_RK4) {
-            prefetch_line(w.lam0 + o);
+            if (w.stage > 0) prefetch_line(w.lam0 + o);
             if (w.stage == 3) {
               prefetch_line(w.f0 + o);
               prefetch_line(w.f1 + o);
@@ -273,10 +279,24 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
     if (!more) chain_release();
     double dsq = 0.0;
     copy_wait<0>();
+    // read last: on its way meanwhile
+    if (L::EPI && w.mode != ADJ_VJP) {
+      copy_rows(ebuf, w.seed, S::NP * 4, E, e0, E);
+      if (w.mode == ADJ_RK4) copy_rows(ebuf + L::STATE, w.lam0, S::NP * 4, E, e0, E);
+      copy_commit();
+    }
     if (more) fetch(b + gridDim.x, wbuf + cur * L::BUF);
     if (__any_sync(0xffffffffu, act)) {
       TileGeo<K, AFF> geo;
       geo.template load<P>(ucol + 2 * L::STATE);
+      const double dte = w.mode == ADJ_RK4 && act ? __ldg(w.dt + e) : 0.0;
+      const double* const ecol = ebuf + (lane >> 2);
+      auto seed_at = [&](int c, int s) {
+        return L::EPI ? ecol[(s * S::NP + 4 * c + l) * 8] : __ldg(w.seed + off + (4 * c * E + s * plane));
+      };
+      auto lam0_at = [&](int c, int s) {
+        return L::EPI ? ecol[L::STATE + (s * S::NP + 4 * c + l) * 8] : w.lam0[off + (4 * c * E + s * plane)];
+      };
       double acc[T::NT][4][2];
 #pragma unroll
       for (int t = 0; t < T::NT; ++t)
@@ -292,68 +312,17 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
 #pragma unroll
         for (int s = 0; s < 4; ++s) lnb[s] = next.oth >= 0 ? __ldg(p + s * plane) : 0.0;
       };
-      neighbour(0);
-#pragma unroll 1
-      for (int fs = 0; fs < T::FS; ++fs) {
-        const AdjFace<K, P> fp = next;
-        const bool valid = fp.k >= 0 && (P == 1 || l < S::NQF);
-        double jt[JAC ? 16 : 1];
+      // the Jacobians are loaded as soon as the registers of the slot before are free
+      double jt[JAC ? 16 : 1];
+      auto jacobian = [&](int fs) {
         if constexpr (JAC) {
+          const bool valid = next.k >= 0 && (P == 1 || l < S::NQF);
           const double* p = w.jac + (e0 / TILE_E) * J::TILE + fs * 16 * J::ROW + (lane >> 2) * J::LPE + l;
 #pragma unroll
           for (int k = 0; k < 16; ++k) jt[k] = valid ? __ldg(p + k * J::ROW) : 0.0;
         }
-        const double bo = fr[T::A_TRO * 32], bn = fr[T::A_TRN * 32];
-        double d[4][2];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          d[s][0] = d[s][1] = 0.0;
-          mma(d[s], fp.own >= 0 ? lcol[(s * S::NP + fp.own) * 8] : 0.0, bo);
-          mma(d[s], lnb[s], bn);
-        }
-        if (fs + 1 < T::FS) neighbour(fs + 1);
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        if constexpr (JAC) {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const double x = d[s][0] - d[s][1];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) a[u] = fma(x, jt[4 * u + s], a[u]);
-          }
-        } else {
-          double t[4][2];
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            t[s][0] = t[s][1] = 0.0;
-            const double o = fp.oth >= 0 ? __ldg(w.U + fp.oth * E + fp.nb + s * plane) : 0.0;
-            mma(t[s], fp.own >= 0 ? ucol[(s * S::NP + fp.own) * 8] : 0.0, bo);
-            mma(t[s], o, bn);
-          }
-          if (valid) {
-            const double* eg = m.edge_geo + 4 * (int64_t)fp.k;
-            const double p_back = (myinst >= 0 && m.inst_p_back) ? __ldg(m.inst_p_back + myinst) : ph.p_back;
-            const double tc[4] = {t[0][0], t[1][0], t[2][0], t[3][0]}, tn[4] = {t[0][1], t[1][1], t[2][1], t[3][1]};
-            Dual<4> F[4];
-            double coef;
-            face_jacobian(tc, tn, fp.code, fp.nb, __ldg(eg), __ldg(eg + 1), __ldg(eg + 2) * fr[T::A_WF * 32], ph, p_back, F,
-                          coef);
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-              const double x = coef * (d[s][0] - d[s][1]);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) a[u] = fma(x, F[s].d[u], a[u]);
-            }
-          }
-          __syncwarp();
-        }
-#pragma unroll
-        for (int t = 0; t < T::NT; ++t) {
-          const double b8 = fr[(T::A_LF + fs * T::NT + t) * 32];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) mma(acc[t][u], a[u], b8);
-        }
-      }
-
+      };
+      neighbour(0);
       // ---- volume: phi_jq (J_F^T cF + J_G^T cG) at every volume point
 #pragma unroll 1
       for (int vt = 0; vt < T::VT; ++vt) {
@@ -422,7 +391,71 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
         }
       }
 
+      // ---- faces
+      jacobian(0);
+#pragma unroll 1
+      for (int fs = 0; fs < T::FS; ++fs) {
+        const AdjFace<K, P> fp = next;
+        const bool valid = fp.k >= 0 && (P == 1 || l < S::NQF);
+        const double bo = fr[T::A_TRO * 32], bn = fr[T::A_TRN * 32];
+        double d[4][2];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          d[s][0] = d[s][1] = 0.0;
+          mma(d[s], fp.own >= 0 ? lcol[(s * S::NP + fp.own) * 8] : 0.0, bo);
+          mma(d[s], lnb[s], bn);
+        }
+        if (fs + 1 < T::FS) neighbour(fs + 1);
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        if constexpr (JAC) {
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            const double x = d[s][0] - d[s][1];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) a[u] = fma(x, jt[4 * u + s], a[u]);
+          }
+          if (fs + 1 < T::FS) jacobian(fs + 1);
+        } else {
+          double t[4][2];
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            t[s][0] = t[s][1] = 0.0;
+            const double o = fp.oth >= 0 ? __ldg(w.U + fp.oth * E + fp.nb + s * plane) : 0.0;
+            mma(t[s], fp.own >= 0 ? ucol[(s * S::NP + fp.own) * 8] : 0.0, bo);
+            mma(t[s], o, bn);
+          }
+          if (valid) {
+            const double* eg = m.edge_geo + 4 * (int64_t)fp.k;
+            const double p_back = (myinst >= 0 && m.inst_p_back) ? __ldg(m.inst_p_back + myinst) : ph.p_back;
+            const double tc[4] = {t[0][0], t[1][0], t[2][0], t[3][0]}, tn[4] = {t[0][1], t[1][1], t[2][1], t[3][1]};
+            Dual<4> F[4];
+            double coef;
+            face_jacobian(tc, tn, fp.code, fp.nb, __ldg(eg), __ldg(eg + 1), __ldg(eg + 2) * fr[T::A_WF * 32], ph, p_back, F,
+                          coef);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+              const double x = coef * (d[s][0] - d[s][1]);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) a[u] = fma(x, F[s].d[u], a[u]);
+            }
+          }
+          __syncwarp();
+        }
+#pragma unroll
+        for (int t = 0; t < T::NT; ++t) {
+          const double b8 = fr[(T::A_LF + fs * T::NT + t) * 32];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mma(acc[t][u], a[u], b8);
+        }
+      }
+
       // ---- epilogue
+      if (L::EPI && w.mode != ADJ_VJP) {
+        if (more)
+          copy_wait<1>();
+        else
+          copy_wait<0>();
+      }
       if (w.mode == ADJ_VJP || w.mode == ADJ_DEFECT) {
 #pragma unroll
         for (int c = 0; c < T::NS; ++c) {
@@ -432,7 +465,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
             const int64_t o = off + (4 * c * E + s * plane);
             double v = acc[c >> 1][s][c & 1];
             if (w.mode == ADJ_DEFECT) {
-              v -= __ldg(w.seed + o);
+              v -= seed_at(c, s);
               dsq = fma(v, v, dsq);
             }
             if (w.out) w.out[o] = v;
@@ -451,8 +484,18 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
 #pragma unroll
           for (int s = 0; s < 4; ++s)
             d[c][s] = act && 4 * c + l < S::NP
-                          ? acc[c >> 1][s][c & 1] - __ldg(w.seed + off + (4 * c * E + s * plane))
+                          ? acc[c >> 1][s][c & 1] - seed_at(c, s)
                           : 0.0;
+        double fsum[T::NS][4];  // last stage: f0 + 2 f1 + 2 f2, loaded ahead of the mass contractions
+        if (w.mode == ADJ_RK4 && w.stage == 3) {
+#pragma unroll
+          for (int c = 0; c < T::NS; ++c)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+              const int64_t o = off + (4 * c * E + s * plane);
+              fsum[c][s] = act && 4 * c + l < S::NP ? __ldg(w.f0 + o) + 2.0 * __ldg(w.f1 + o) + 2.0 * __ldg(w.f2 + o) : 0.0;
+            }
+        }
         auto apply = [&](int table) {
           __syncwarp();
 #pragma unroll
@@ -484,7 +527,6 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
           apply(T::A_MT);
         }
         if (act) {
-          const double dte = w.mode == ADJ_RK4 ? __ldg(w.dt + e) : 0.0;
 #pragma unroll
           for (int c = 0; c < T::NS; ++c) {
             if (4 * c + l >= S::NP) continue;
@@ -496,15 +538,15 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
                 w.out[o] = rr;
               } else if (w.stage == 0) {
                 w.f0[o] = rr;
-                w.out[o] = w.lam0[o] + 0.5 * dte * rr;
+                w.out[o] = lam0_at(c, s) + 0.5 * dte * rr;
               } else if (w.stage == 1) {
                 w.f1[o] = rr;
-                w.out[o] = w.lam0[o] + 0.5 * dte * rr;
+                w.out[o] = lam0_at(c, s) + 0.5 * dte * rr;
               } else if (w.stage == 2) {
                 w.f2[o] = rr;
-                w.out[o] = w.lam0[o] + dte * rr;
+                w.out[o] = lam0_at(c, s) + dte * rr;
               } else {
-                w.lam0[o] = w.lam0[o] + dte / 6.0 * (w.f0[o] + 2.0 * w.f1[o] + 2.0 * w.f2[o] + rr);
+                w.lam0[o] = lam0_at(c, s) + dte / 6.0 * (fsum[c][s] + rr);
               }
             }
           }
