@@ -48,6 +48,10 @@ struct Tile {
   using S = Shape<K, P>;
   static constexpr int NS = (S::NP + 3) / 4;   // node slots
   static constexpr int NT = (NS + 1) / 2;      // node tiles (two slots each)
+  // Where the last node tile holds one or two nodes (of eight columns), they are summed by multiply-adds
+  // in the lanes that hold the points, and over the lanes once at the end: REM nodes, MTS tiles by mma.
+  static constexpr int REM = NS % 2 == 1 && NS > 1 && S::NP - 8 * (NT - 1) <= 2 ? S::NP - 8 * (NT - 1) : 0;
+  static constexpr int MTS = REM ? NT - 1 : NT;
   static constexpr int VS = (S::NQV + 3) / 4;  // volume-point slots
   static constexpr int VT = (VS + 1) / 2;
   static constexpr int FPS = P == 1 ? 2 : 1;   // faces per face-point slot
@@ -325,6 +329,36 @@ __device__ __forceinline__ void mma(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
+}
+
+// The remaining nodes of a contraction (Tile::REM): this lane's share of node 8 MTS + r from its own item
+// of the k-step is x times entry (k = l, column of that node) of the fragment, at row[8 r].
+template <int K, int P, int N>
+__device__ __forceinline__ void remainder(double (&rem)[N][4], const double* row, const double (&x)[4]) {
+#pragma unroll
+  for (int r = 0; r < Tile<K, P>::REM; ++r) {
+    const double b = row[8 * r];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) rem[r][s] = fma(b, x[s], rem[r][s]);
+  }
+}
+// ... summed over the four lanes (a product with a matrix of ones) into the last tile's first slot.
+template <int K, int P, int N>
+__device__ __forceinline__ void remainder_sum(double (&acc)[Tile<K, P>::NT][4][2], const double (&rem)[N][4], int l) {
+  using T = Tile<K, P>;
+  if constexpr (T::REM > 0) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      double v = 0.0;
+#pragma unroll
+      for (int r = 0; r < T::REM; ++r) {
+        double d[2] = {0.0, 0.0};
+        mma(d, rem[r][s], 1.0);
+        v = l == r ? d[0] : v;
+      }
+      acc[T::NT - 1][s][0] = v;
+    }
+  }
 }
 
 // Sum, maximum and minimum over an element's four lanes (every lane gets it; the

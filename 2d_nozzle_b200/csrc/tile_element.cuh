@@ -559,6 +559,12 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
         for (int t = 0; t < T::NT; ++t)
 #pragma unroll
           for (int s = 0; s < 4; ++s) acc[t][s][0] = acc[t][s][1] = 0.0;
+        double rem[T::REM ? T::REM : 1][4];
+#pragma unroll
+        for (int r = 0; r < T::REM; ++r)
+#pragma unroll
+          for (int s = 0; s < 4; ++s) rem[r][s] = 0.0;
+        const double* const frl = fr - lane + l;  // entry (k = l, n = 2 r) of fragment n is frl[32 n + 8 r]
 
         // ---- volume
         copy_wait<1>();
@@ -608,12 +614,16 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
               fe[s] = (a10 * F[s] + a11 * G[s]) * vs;
             }
 #pragma unroll
-            for (int t = 0; t < T::NT; ++t) {
+            for (int t = 0; t < T::MTS; ++t) {
               const double bx = fr[T::vx(fo, v, t, 0) * 32], be = fr[T::vx(fo, v, t, 1) * 32];
 #pragma unroll
               for (int s = 0; s < 4; ++s) mma(acc[t][s], fx[s], bx);
 #pragma unroll
               for (int s = 0; s < 4; ++s) mma(acc[t][s], fe[s], be);
+            }
+            if constexpr (T::REM > 0) {
+              remainder<K, P>(rem, frl + T::vx(fo, v, T::NT - 1, 0) * 32, fx);
+              remainder<K, P>(rem, frl + T::vx(fo, v, T::NT - 1, 1) * 32, fe);
             }
           }
         }
@@ -666,11 +676,12 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
           }
           __syncwarp();
 #pragma unroll
-          for (int t = 0; t < T::NT; ++t) {
+          for (int t = 0; t < T::MTS; ++t) {
             const double b8 = fr[T::lf(fo, fs, t) * 32];
 #pragma unroll
             for (int s = 0; s < 4; ++s) mma(acc[t][s], F[s], b8);
           }
+          if constexpr (T::REM > 0) remainder<K, P>(rem, frl + T::lf(fo, fs, T::NT - 1) * 32, F);
           // wave = sum over faces of the largest signal speed times the length; a NaN speed does
           // not count, as in the one-thread kernel
           double sm = sp > 0.0 ? sp : 0.0;
@@ -684,6 +695,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
           }
         }
         if (w.wave && act && l == 0) w.wave[e] = wave;
+        remainder_sum<K, P>(acc, rem, l);
 
         // ---- quadrilaterals' rates: acc holds Phi^-1 R; -Phi^-T (acc / (w det))
         if (K == 1 && rate) {
@@ -701,15 +713,22 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
           for (int t = 0; t < T::NT; ++t)
 #pragma unroll
             for (int s = 0; s < 4; ++s) acc[t][s][0] = acc[t][s][1] = 0.0;
+#pragma unroll
+          for (int r = 0; r < T::REM; ++r)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) rem[r][s] = 0.0;
           __syncwarp();
 #pragma unroll
-          for (int c = 0; c < T::NS; ++c)
+          for (int c = 0; c < T::NS; ++c) {
 #pragma unroll
-            for (int t = 0; t < T::NT; ++t) {
+            for (int t = 0; t < T::MTS; ++t) {
               const double b8 = fr[(T::MT + c * T::NT + t) * 32];
 #pragma unroll
               for (int s = 0; s < 4; ++s) mma(acc[t][s], y[c][s], b8);
             }
+            if constexpr (T::REM > 0) remainder<K, P>(rem, frl + (T::MT + c * T::NT + T::NT - 1) * 32, y[c]);
+          }
+          remainder_sum<K, P>(acc, rem, l);
         }
 
         if (!stage) {
