@@ -11,7 +11,8 @@
 // With the Superbee limiter (limiter 2) the element kernel leaves the stage
 // unlimited and three passes follow (cell means, their maximum -- per
 // instance in a batch -- and the slope limiter with the positivity limiter);
-// the tile kernel forms the means and maxima itself, so one follows it.
+// the tile kernel forms the means and maxima itself, so one follows it (2 240
+// quadratic triangles, a stage: 24 -> 17 us), except under a block list.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -85,19 +86,21 @@ cudaError_t launch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cuda
   if constexpr (P > 0) {
     if (m.split == TILE_LANES) {
       const int64_t blocks = m.fwd_blocks ? m.n_fwd_blocks : (m.n_elem + TILE_EB - 1) / TILE_EB;
-      // Superbee: the stage kernel leaves the averages and, from zero, their maxima; one pass follows
+      // Superbee: the stage kernel leaves the averages and, from zero, their maxima; one pass follows.
+      // Under a block list it sees only the listed elements, so the averages keep their own passes.
       Work wt = w;
-      if (sb) {
+      const bool fused = sb && !m.fwd_blocks;
+      if (sb) wt.chained = false;
+      if (fused) {
         const cudaError_t e = cudaMemsetAsync(m.lim_scale, 0, sizeof(double) * 4 * (m.elem_inst ? m.n_inst : 1), st);
         if (e != cudaSuccess) return e;
-        wt.chained = false;
       }
       if (blocks > 0) {  // an empty block list: nothing marches
         const cudaError_t e = lim ? launch_tile<K, P, AFF, true>(m, ph, wt, blocks, st)
                                   : launch_tile<K, P, AFF, false>(m, ph, wt, blocks, st);
         if (e != cudaSuccess) return e;
       }
-      if (sb) return blocks > 0 ? tile_superbee<K, P, AFF>(m, ph, w.out, w.out, w.counters, w.flags, true, st) : cudaSuccess;
+      if (fused) return tile_superbee<K, P, AFF>(m, ph, w.out, w.out, w.counters, w.flags, true, st);
       done = true;
     }
   }

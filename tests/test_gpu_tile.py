@@ -82,6 +82,40 @@ def test_superbee_tiles_agree_with_one_thread(cuda, kind, p, nx, nr):
 
 @pytest.mark.parametrize("kind", ["tri", "quad"])
 @pytest.mark.parametrize("p", [1, 2, 3])
+def test_superbee_under_a_block_list(cuda, kind, p):
+    """A stage that lists the first 128 elements only: the slope limiter still takes every element's
+    average, from its own pass, as it does after the one-thread kernel with the same elements listed."""
+    import ctypes as C
+
+    import torch
+
+    capi, cfg, mesh = pkg("capi"), pkg("config"), pkg("mesh")
+    topo, xf, rf = mesh.channel_topology(kind, nx=33, nr=11)
+    X = mesh.rectangle_coords(xf, rf)
+    X = X + 0.003 * np.sin(7.0 * X[:, ::-1])
+    ops = pkg("operators").build_operators(topo, X, p, lean=True)
+    U = _states(ops, 7)
+    bk = pkg("backend").B200Backend(ops, cfg.FlowConditions(flux="roe"),
+                                   cfg.SolverOptions(cfl=0.5, limiter="superbee", tvb_constant=1.0), device_metrics=True)
+    src = bk.mesh.pack(U, torch.empty(4 * bk.mesh.np_ * bk.mesh.E, dtype=torch.float64, device="cuda"))
+    out = []
+    for name in ("t1", "split4"):
+        pkg("autotune").apply_variant(bk.mesh, name)
+        mc = capi.Mesh()
+        C.memmove(C.byref(mc), bk.mesh.c_ref, C.sizeof(capi.Mesh))
+        listed = torch.arange(128 // int(bk.lib.nzb_block_width(C.byref(mc), 0)), dtype=torch.int32, device="cuda")
+        mc.fwd_blocks, mc.n_fwd_blocks = listed.data_ptr(), listed.numel()
+        bk.mesh.lim_means.fill_(1e3)
+        new, dt = src.clone(), torch.ones(bk.mesh.E, dtype=torch.float64, device="cuda")
+        a = capi.StageArgs()
+        a.V, a.out, a.dt, a.dt_factor, a.a, a.b, a.stage = src.data_ptr(), new.data_ptr(), dt.data_ptr(), 0.1, 0.0, 1.0, 1
+        capi.check(bk.lib.nzb_stage(C.byref(mc), bk._phys_ref, C.byref(a), bk._stream), "nzb_stage")
+        out.append(new.cpu().numpy())
+    assert rel(out[1], out[0]) < TOL
+
+
+@pytest.mark.parametrize("kind", ["tri", "quad"])
+@pytest.mark.parametrize("p", [1, 2, 3])
 @pytest.mark.parametrize("nx,nr", [s for s in SIZES if s != (160, 97)] + [(72, 100)])
 def test_adjoint_tiles_agree_with_one_thread(cuda, kind, p, nx, nr, monkeypatch):
     """The product, the rate (both differentiate the fluxes in the kernel) and a run of three RK4 steps
