@@ -255,6 +255,17 @@ def ResidualFunction(model: AdjointModel, U_soa, X, p_back):
     return _Residual.apply(model, U_soa, X, p_back)
 
 
+def _jacobian_workspace(lib, mesh, device):
+    """The face Jacobians' workspace of an adjoint march, or None where its kernel uses none or memory is
+    short (the products then differentiate in place).  From torch's allocator: a new linearisation
+    reuses the last one's memory instead of mapping its own (165 MB at 143 360 quadratic triangles)."""
+    n = lib.nzb_adjoint_jacobian_doubles(C.byref(mesh))
+    try:
+        return torch.empty(n, dtype=torch.float64, device=device) if n > 0 else None
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 class AdjointMarch:
     """The adjoint pseudo-time march of one linearisation, as one device object."""
 
@@ -306,6 +317,9 @@ class AdjointMarch:
                                                      offs.ctypes.data, C.byref(am), C.byref(h)), "nzb_adjoint_create")
         self.am = am
         self.handle = h.value
+        self.jac = _jacobian_workspace(self.model.lib, self.model.mesh.c, self.model.device)
+        capi.check(self.model.lib.nzb_adjoint_jacobians(h, 0, self.jac.data_ptr() if self.jac is not None else None),
+                   "nzb_adjoint_jacobians")
 
     def __del__(self):
         if getattr(self, "handle", None):
@@ -742,6 +756,7 @@ class BatchGradient:
         offs = np.zeros(1, np.int64)
         elem_count = np.asarray([hi - lo for lo, hi in spans], np.int64)
         handles = {}  # adjoint march object -> its block list (kept alive with it)
+        jac = []  # the face Jacobians' workspace, one for the objects that follow one another
 
         def variant_mesh(context):
             mc = capi.Mesh()
@@ -767,6 +782,10 @@ class BatchGradient:
             hh = capi.P()
             capi.check(lib.nzb_adjoint_create(1, C.byref(mc), C.byref(ph), C.byref(bf), offs.ctypes.data,
                                               C.byref(am), C.byref(hh)), "nzb_adjoint_create")
+            if not jac and lib.nzb_adjoint_jacobian_doubles(C.byref(mc)) > 0:
+                jac.append(_jacobian_workspace(lib, mc, dev))
+            capi.check(lib.nzb_adjoint_jacobians(hh, 0, jac[0].data_ptr() if jac and jac[0] is not None else None),
+                       "nzb_adjoint_jacobians")
             handles[hh.value] = keep
             return hh.value, int(blocks.size)
 

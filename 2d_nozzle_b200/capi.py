@@ -315,6 +315,8 @@ SIGNATURES = [
     ("nzb_local_dt", C.c_int, [C.POINTER(Mesh), P, C.c_double, P, P]),
     ("nzb_adjoint_create", C.c_int, [C.c_int, C.POINTER(Mesh), C.POINTER(Physics), C.POINTER(AdjointBuffers), P,
                                      C.POINTER(AdjointMarch), C.POINTER(P)]),
+    ("nzb_adjoint_jacobian_doubles", I64, [C.POINTER(Mesh)]),
+    ("nzb_adjoint_jacobians", C.c_int, [P, C.c_int, P]),
     ("nzb_adjoint_run", C.c_int, [P, C.c_int, P]),
     ("nzb_adjoint_destroy", C.c_int, [P]),
 ]

@@ -78,7 +78,7 @@ static int block_threads(int kind, int order) {
   }
   return 128;
 }
-// Elements per block of the forward element kernel: 32 with four threads per
+// Elements per block of the forward element kernel: 32 with four lanes per
 // element, else one per thread.
 static int element_width(const nzb_mesh& m) {
   return (m.split == TILE_LANES && m.order > 0) ? TILE_EB : block_threads(m.kind, m.order);
@@ -591,7 +591,8 @@ struct AdjBatch {
   cudaEvent_t fork = nullptr;
   // per bucket: room for its face Jacobians, formed at the start of every run (null: a variant
   // without them, or no memory for them -- then every product differentiates the fluxes itself)
-  std::vector<double*> jac;
+  std::vector<double*> jac;   // face Jacobians of the run (null: the products differentiate in place)
+  std::vector<char> jac_set;  // 0: nobody decided yet, 1: the caller's (or none), 2: our own
   std::map<int, cudaGraphExec_t> graphs;  // key: steps per chunk
 };
 
@@ -1301,25 +1302,50 @@ int nzb_adjoint_create(int n_buckets, const nzb_mesh* meshes, const nzb_physics*
       nzb_adjoint_destroy(reinterpret_cast<nzb_adjoint*>(A));
       return -1;
     }
-    const nzb_mesh& m = A->mesh[b];
-    const int64_t n = m.vjp_split != TILE_LANES ? 0
-                      : m.kind == NZB_TRI       ? vjp_jac_doubles_tri(m.order, m.n_elem)
-                                                : vjp_jac_doubles_quad(m.order, m.n_elem);
+    A->jac.push_back(nullptr);
+    A->jac_set.push_back(0);
+  }
+  *out = reinterpret_cast<nzb_adjoint*>(A);
+  return 0;
+}
+
+int64_t nzb_adjoint_jacobian_doubles(const nzb_mesh* mesh) {
+  if (!mesh || mesh->vjp_split != TILE_LANES || mesh->order < 1 || mesh->n_elem < 1) return 0;
+  return mesh->kind == NZB_TRI ? vjp_jac_doubles_tri(mesh->order, mesh->n_elem)
+                               : vjp_jac_doubles_quad(mesh->order, mesh->n_elem);
+}
+
+int nzb_adjoint_jacobians(nzb_adjoint* adjoint, int bucket, double* jac) {
+  AdjBatch* A = reinterpret_cast<AdjBatch*>(adjoint);
+  if (!A) return fail("adjoint is null");
+  if (bucket < 0 || bucket >= (int)A->mesh.size()) return fail("adjoint_jacobians: no such bucket");
+  if (A->jac_set[bucket]) return fail("adjoint_jacobians: already decided (call it once, before the first run)");
+  if ((uintptr_t)jac & 15) return fail("adjoint_jacobians: the workspace must be 16-byte aligned");
+  A->jac[bucket] = nzb_adjoint_jacobian_doubles(&A->mesh[bucket]) > 0 ? jac : nullptr;
+  A->jac_set[bucket] = 1;
+  return 0;
+}
+
+// A march whose caller gave no workspace takes its own at its first run of steps.
+static void own_jacobians(AdjBatch& A) {
+  for (size_t b = 0; b < A.mesh.size(); ++b) {
+    if (A.jac_set[b]) continue;
+    const int64_t n = nzb_adjoint_jacobian_doubles(&A.mesh[b]);
     double* jac = nullptr;
     if (n > 0 && cudaMalloc(&jac, sizeof(double) * n) != cudaSuccess) {
       cudaGetLastError();  // not enough memory: the products work without
       jac = nullptr;
     }
-    A->jac.push_back(jac);
+    A.jac[b] = jac;
+    A.jac_set[b] = 2;
   }
-  *out = reinterpret_cast<nzb_adjoint*>(A);
-  return 0;
 }
 
 int nzb_adjoint_run(nzb_adjoint* adjoint, int n_steps, void* stream) {
   AdjBatch* A = reinterpret_cast<AdjBatch*>(adjoint);
   if (!A) return fail("adjoint is null");
   if (n_steps < 0) return fail("adjoint_run: n_steps must be >= 0");
+  if (n_steps > 0) own_jacobians(*A);
   cudaStream_t caller = (cudaStream_t)stream;
   if (cuda_check(cudaEventRecord(A->ev_in, caller), "event record") ||
       cuda_check(cudaStreamWaitEvent(A->stream, A->ev_in, 0), "stream wait"))
@@ -1337,8 +1363,8 @@ int nzb_adjoint_destroy(nzb_adjoint* adjoint) {
   AdjBatch* A = reinterpret_cast<AdjBatch*>(adjoint);
   if (!A) return 0;
   for (auto& kv : A->graphs) cudaGraphExecDestroy(kv.second);
-  for (double* p : A->jac)
-    if (p) cudaFree(p);
+  for (size_t b = 0; b < A->jac.size(); ++b)
+    if (A->jac[b] && A->jac_set[b] == 2) cudaFree(A->jac[b]);
   if (A->ev_in) cudaEventDestroy(A->ev_in);
   if (A->ev_out) cudaEventDestroy(A->ev_out);
   if (A->fork) cudaEventDestroy(A->fork);

@@ -82,7 +82,9 @@ enum { NZB_OP_RESIDUAL = 0, NZB_OP_RATE = 1 };
  * three passes after the element kernel -- cell averages, their maximum per
  * instance (lim_scale holds 4 per instance: n_inst of them with elem_inst, one
  * without), the slope limiter with the positivity limiter -- and count an
- * element as scaled when either limiter changed it.  elem_share is each
+ * element as scaled when either limiter changed it.  A stage with split = 4 and
+ * no block list leaves the averages and maxima itself, so only the last pass
+ * follows.  elem_share is each
  * element's area over its own instance's domain area.
  * edge_pass = 1 splits every residual / stage into two launches: one thread
  * per edge evaluates each edge's fluxes once (the reference's edge_pass), then
@@ -90,15 +92,13 @@ enum { NZB_OP_RESIDUAL = 0, NZB_OP_RATE = 1 };
  * element kernel, from both sides.  Both evaluate the same formulas and agree
  * to round-off (the compiler may contract multiply-adds differently); which is
  * faster depends on the element kind, order and mesh size.
- * split = 4 (orders >= 1) runs the element kernel with four threads per
- * element -- faces and volume points split over a block's four warps, the
- * projection by component, the limiter's probe points split -- and ignores
- * edge_pass; split = 0 or 1 runs one thread per element.  It agrees with the
- * one-thread kernels to round-off (a few sums associate differently).
- * vjp_split = 4 (orders >= 1) runs the adjoint state kernel the same way:
- * faces and volume points split over four warps, each warp gathering one
- * component of every node in the one-thread kernel's order; it agrees with
- * the one-thread kernel to round-off.
+ * split = 4 (orders >= 1) runs the element kernel with four lanes of a warp
+ * per element and its contractions on the FP64 tensor cores, and ignores
+ * edge_pass and minv; split = 0 or 1 runs one thread per element.  It agrees
+ * with the one-thread kernels to round-off (sums associate differently).
+ * vjp_split = 4 (orders >= 1) runs the adjoint state kernel the same way; a run
+ * of adjoint steps (nzb_adjoint_run) then forms the face Jacobians of its frozen
+ * state once, in a workspace (nzb_adjoint_jacobians), and its products read them.
  */
 typedef struct {
   int32_t kind;
@@ -418,6 +418,14 @@ typedef struct nzb_adjoint nzb_adjoint;
 int nzb_adjoint_create(int n_buckets, const nzb_mesh* meshes, const nzb_physics* phys,
                        const nzb_adjoint_buffers* buffers, const int64_t* elem_offset,
                        const nzb_adjoint_march* march, nzb_adjoint** out);
+/* The workspace of a bucket's face Jacobians (nzb_mesh.vjp_split = 4): its size in
+ * doubles (0: the bucket's kernel uses none), and the caller's choice of it, once
+ * and before the first run: 16-byte aligned, kept alive until the march is
+ * destroyed, shared at will between marches whose runs follow one another on one
+ * stream (each run forms its Jacobians anew); null: the products differentiate in
+ * place.  A march without a choice allocates its own at its first run of steps. */
+int64_t nzb_adjoint_jacobian_doubles(const nzb_mesh* mesh);
+int nzb_adjoint_jacobians(nzb_adjoint* adjoint, int bucket, double* jac);
 int nzb_adjoint_run(nzb_adjoint* adjoint, int n_steps, void* stream);
 int nzb_adjoint_destroy(nzb_adjoint* adjoint);
 

@@ -143,6 +143,39 @@ def test_adjoint_tiles_agree_with_one_thread(cuda, kind, p, nx, nr, monkeypatch)
         assert rel(y.cpu().numpy(), x.cpu().numpy()) < TOL
 
 
+@pytest.mark.parametrize("kind", ["tri", "quad"])
+@pytest.mark.parametrize("p", [1, 3])
+def test_adjoint_march_with_any_workspace(cuda, kind, p, monkeypatch):
+    """A run of RK4 steps with the caller's Jacobian workspace, with the march's own (the same bits) and
+    with none (the products differentiate in place); the choice is made once."""
+    import ctypes as C
+
+    import torch
+
+    ad, capi, cfg, mesh = pkg("adjoint"), pkg("capi"), pkg("config"), pkg("mesh")
+    topo, xf, rf = mesh.channel_topology(kind, nx=11, nr=3)
+    ops = pkg("operators").build_operators(topo, mesh.rectangle_coords(xf, rf), p)
+    m = ad.AdjointModel(ops, cfg.FlowConditions(flux="ausmup"), cfg.SolverOptions(cfl=0.5))
+    u = ad.to_soa(torch.as_tensor(_states(ops, 8), device="cuda"))
+    sd = ad.to_soa(torch.as_tensor(np.random.default_rng(9).standard_normal((ops.n_elem, ops.ref.n_basis, 4)), device="cuda"))
+    out = []
+    for given in (True, False):
+        if not given:
+            monkeypatch.setattr(ad, "_jacobian_workspace", lambda *a: None)
+        am = ad.AdjointMarch(m, u, sd, 0.5)
+        out.append(am.solve(tolerance=0.0, max_iterations=3, check_interval=3)[0].clone())
+        with pytest.raises(capi.NativeError, match="once"):
+            capi.check(m.lib.nzb_adjoint_jacobians(am.handle, 0, None), "nzb_adjoint_jacobians")
+    offs, h = np.zeros(1, np.int64), capi.P()
+    capi.check(m.lib.nzb_adjoint_create(1, m.mesh.c_ref, C.byref(am.ph), C.byref(am.bf), offs.ctypes.data, C.byref(am.am),
+                                        C.byref(h)), "nzb_adjoint_create")
+    m.lib.nzb_adjoint_destroy(am.handle)
+    am.handle = h.value
+    own = am.solve(tolerance=0.0, max_iterations=3, check_interval=3)[0]
+    assert torch.equal(own, out[0])
+    assert rel(out[1].cpu().numpy(), out[0].cpu().numpy()) < TOL
+
+
 @pytest.mark.parametrize("decade", [-30, -20, -10, -1, 0, 1, 10, 20, 29])
 def test_reciprocals_are_accurate(cuda, decade):
     """1 / a and 1 / sqrt(a) of the fluxes against the division's and torch's.  The step's remainder is
