@@ -6,21 +6,20 @@ The forward kernels come in three variants:
                   both sides inside the element kernel;
 * ``t1_edge``  -- one thread per element, the fluxes from a separate edge
                   pass (one thread per edge, each flux once);
-* ``split4``   -- four threads per element (a block of four warps owns 32
-                  elements: faces and volume points split over the warps, the
-                  projection by component, the limiter's probe scan split).
+* ``split4``   -- four lanes of a warp per element, the contractions on the
+                  FP64 tensor cores (``csrc/tile_element.cuh``).
 
 They evaluate the same formulas and agree to round-off on a step (the
 compiler contracts multiply-adds differently in different kernels, and
-``split4`` associates a few sums differently).  The adjoint state kernel has
+``split4`` associates sums differently).  The adjoint state kernel has
 ``t1`` and ``split4`` too.
 
 Which is fastest can depend on the context, so the table has two: ``single``
 (one solve on its own mesh of a few thousand elements -- latency-bound) and
 ``batch`` (a bucket of a batch marching beside the other buckets, or one mesh
 that fills the GPU -- throughput-bound).  ``split4`` is the forward choice of
-both above p = 0: a stage of a single solve takes 7-18 us with it and 25-220 us
-with one thread per element, a step of a 72-member sweep (211 680 elements) 0.55
+both above p = 0: a stage of a single solve takes 7-14 us with it and 25-220 us
+with one thread per element, a step of a 72-member sweep (211 680 elements) 0.49
 against 1.0 ms.  Within a context the variant is fixed per (kind, order), never
 per mesh; a batch built with ``variants="single"`` runs the plain solve's kernels
 and gives its bits.  One exception, :func:`bucket_context`.
@@ -107,7 +106,7 @@ def variant_for(kind: str, order: int, context: str = "single") -> str:
     if context == "lone":
         return "t1"
     name = _lookup(kind, order, context, "fwd")
-    # four threads per element apply from p = 1 up
+    # four lanes per element apply from p = 1 up
     return "t1" if (name == "split4" and int(order) == 0) else name
 
 
@@ -117,7 +116,7 @@ def apply_variant(mesh, name: str) -> None:
     mesh.edge_pass = v["edge_pass"]
 
 
-# The adjoint state kernel: one thread per element (``t1``) or four (``split4``),
+# The adjoint state kernel: one thread per element (``t1``) or four lanes (``split4``),
 # chosen per (kind, order) and context from the same table; NZB_VJP_VARIANT
 # forces one.
 VJP_VARIANTS = {"t1": 1, "split4": 4}
@@ -169,12 +168,11 @@ LONE_ELEMENTS = 16384
 
 def bucket_context(n_instances: int, n_elem: int, variants: str) -> str:
     """The variant context of a batch's bucket: ``variants``, except that a throughput bucket holding a
-    single large instance takes ``lone``, whose forward choice is the one-thread kernel.  That is the
-    stage benchmark's shape -- one large mesh of random states, half of whose elements the limiter
-    rescales toward vacuum -- and a step from such states magnifies the last bits of the fluxes by up to
-    1e8 (a contact speed equal to a wave speed but for round-off), so its results are kept bit for bit
-    although the tile kernel is faster there (500 000 cubic triangles: a limited stage 1.03 against
-    0.62 ms).  Sweeps' instances are far below the line (9 000 elements at refinement 3)."""
+    single large instance takes ``lone``, whose forward choice is the one-thread kernel.  One large mesh
+    of random states, half of whose elements the limiter rescales toward vacuum, magnifies the last bits
+    of the fluxes by up to 1e8 in one step (a contact speed equal to a wave speed but for round-off), so
+    such a batch keeps its results bit for bit although the tile kernel is faster there (500 000 cubic
+    triangles: a limited stage 1.03 against 0.55 ms).  Sweeps' instances are far below the line (9 000 elements at refinement 3)."""
     return "lone" if variants == "batch" and n_instances == 1 and n_elem > LONE_ELEMENTS else variants
 
 

@@ -33,7 +33,7 @@
 //
 // What bounds it: FP64 latency and issue at 12 warps per SM (168 registers; four
 // blocks at 128 spill and are slower at p >= 2: 436 against 380 us at 480 000
-// cubic triangles).  An SM sub-partition's FP64 unit does 16 multiply-adds a cycle
+// cubic triangles when that was tried, before the lean reciprocals).  An SM sub-partition's FP64 unit does 16 multiply-adds a cycle
 // either way, but one mma keeps it busy 16 cycles from one instruction (measured
 // 32.8 TFLOP/s from four warps per SM, where multiply-adds reach 24), so the
 // contractions no longer need warps to hide their latency nor instruction issue.
@@ -41,13 +41,13 @@
 // Measured on a B200, HLLC stage 2 with the limiter quiet / limiting about half of
 // the elements, against the one-thread kernel (k_element) and the block-of-four-
 // warps kernel it replaces where that was in use (us per launch):
-//   480 000 triangles      p = 1  197 / 228 (t1 257 / 286)   p = 2  286 / 422 (423 / 503)
-//                          p = 3  380 / 582 (784 / 1000)
-//   240 000 quadrilaterals p = 1  113 / 127 (202 / 222)      p = 2  243 / 319 (443 / 499)
-//                          p = 3  291 / 410 (1240 / 1408)
-// and inside a march, per stage: 140 triangles p = 1 10.9 -> 7.4, 2 240 triangles
-// p = 2 14.4 -> 9.6, 4 480 quadrilaterals p = 3 44.2 -> 15.3.  The residual of 10^6
-// cubic triangles 776 -> 601 us.
+//   480 000 triangles      p = 1  176 / 207 (t1 257 / 286)   p = 2  260 / 385 (423 / 503)
+//                          p = 3  325 / 530 (784 / 1000)
+//   240 000 quadrilaterals p = 1  100 / 116 (202 / 222)      p = 2  196 / 264 (443 / 499)
+//                          p = 3  262 / 369 (1240 / 1408)
+// and inside a march, per stage: 140 triangles p = 1 10.9 -> 6.8, 2 240 triangles
+// p = 2 14.4 -> 8.7, 4 480 quadrilaterals p = 3 44.2 -> 14.0.  The residual of 10^6
+// cubic triangles 776 -> 540 us.
 #pragma once
 #include "flux.cuh"
 #include "slope.cuh"

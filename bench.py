@@ -172,6 +172,7 @@ def microbench(torch, lib_capi, B, cfg, peak_gbs, peak_kind, nx=1000, nr=500, ki
     results = {}
     for flux in ("roe", "hllc", "ausmup"):
         bk = B(ops, cfg.FlowConditions(flux=flux), cfg.SolverOptions(cfl=0.5), device_metrics=kind != "tri")
+        tiles = bk.mesh.split == 4
         bk.mesh.pack(U, bk._S[0])
         st = torch.cuda.current_stream()
         ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
@@ -228,7 +229,8 @@ def microbench(torch, lib_capi, B, cfg, peak_gbs, peak_kind, nx=1000, nr=500, ki
     n_edge = ops.n_edges_total
     nf = 3 if kind == "tri" else 4
     geo = 40 if kind == "tri" else 2 * nf * 8  # the residual applies no inverse mass
-    minv = 0 if kind == "tri" else NP * NP * 8  # general geometry: per-element inverse mass, read by rates and stages
+    # general geometry: per-element inverse mass, read by the one-thread kernels' rates and stages
+    minv = 0 if kind == "tri" or tiles else NP * NP * 8
     base = geo + 12 * nf + 32.0 * n_edge / E
     alg = {"residual": 2 * S + base + 8, "stage1": 2 * S + base + minv + 8 + 8,
            "stage23": 3 * S + base + minv + 8 + 8}
@@ -238,7 +240,9 @@ def microbench(torch, lib_capi, B, cfg, peak_gbs, peak_kind, nx=1000, nr=500, ki
     # FP64 operations per element (2 per DFMA, 1 per DADD or DMUL thread instruction; divisions and square
     # roots count as the instructions they compile to), counted by ncu on 490,000 cubic triangles and 245,000
     # cubic quadrilaterals of the same state distribution with the one-thread kernels (the stages' counts
-    # depend on how many elements the limiter works on, 53 % / 66 % here)
+    # depend on how many elements the limiter works on, 53 % / 66 % here).  The tile kernel executes more,
+    # its tiles' padding included (2 per DFMA, 512 per FP64 mma: 10178 a cubic triangle's residual, 15371,
+    # 15250 and 15244 its stages); the work without padding is what counts as achieved
     fp64 = {("tri", 3): {"residual_roe": 9067.1, "residual_hllc": 9323.5, "residual_ausmup": 8753.7,
                          "stage1_hllc": 12996.2, "stage2_hllc": 12945.0, "stage3_hllc": 12938.8},
             ("quad", 3): {"residual_roe": 13154.5, "residual_hllc": 13496.5, "residual_ausmup": 12721.2,
@@ -250,10 +254,10 @@ def microbench(torch, lib_capi, B, cfg, peak_gbs, peak_kind, nx=1000, nr=500, ki
             out["kernels"][name]["fp64_tflops"] = fp64[name] * E / t / 1e12
     dom = max(results, key=results.get)
     k = out["kernels"][dom]
-    # DRAM bytes per element of each kernel from an ncu capture of 490,000 cubic triangles
-    # (profiles/k_element_stage_tri_p3_490k.md), scaled to this launch by its element count
-    traffic = ({"residual_roe": 1055.0, "stage1_hllc": 1139.0, "stage2_hllc": 1510.0, "stage3_hllc": 1446.0}
-               if (kind, order) == ("tri", 3) else {})
+    # DRAM bytes per element of the tile kernel from an ncu capture of 490,000 cubic triangles
+    # (profiles/k_tile_p3_stages.md), scaled to this launch by its element count
+    traffic = ({"residual_hllc": 1061.0, "stage1_hllc": 1066.0, "stage2_hllc": 1390.0, "stage3_hllc": 1379.0}
+               if (kind, order) == ("tri", 3) and tiles else {})
     out["roofline"] = {"bound": "hbm", "kernel": dom, "achieved": k["gbs"], "peak": peak_gbs, "unit": "GB/s",
                        "frac": k["gbs"] / peak_gbs, "peak_source": peak_kind,
                        "traffic": traffic[dom] * E if dom in traffic else None,
