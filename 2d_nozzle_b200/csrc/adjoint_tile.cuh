@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
         next.set(mycode, mynb, myk, fs, lane);
         const double* p = w.lam + (next.oth >= 0 ? next.oth * E + next.nb : 0);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) lnb[s] = next.oth >= 0 ? __ldg(p + s * plane) : 0.0;
+        for (int s = 0; s < 4; ++s) lnb[s] = next.oth >= 0 ? p[s * plane] : 0.0;  // the chain's: an ordinary load (tile.cuh)
       };
       // the Jacobians are loaded as soon as the registers of the slot before are free
       double jt[JAC ? 16 : 1];
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileVjpSmem<K, P, AFF, JAC>:
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
               const int64_t o = off + (4 * c * E + s * plane);
-              fsum[c][s] = act && 4 * c + l < S::NP ? __ldg(w.f0 + o) + 2.0 * __ldg(w.f1 + o) + 2.0 * __ldg(w.f2 + o) : 0.0;
+              fsum[c][s] = act && 4 * c + l < S::NP ? w.f0[o] + 2.0 * w.f1[o] + 2.0 * w.f2[o] : 0.0;
             }
         }
         auto apply = [&](int table) {

@@ -98,8 +98,8 @@ __device__ __forceinline__ double warp_min(double v) {
   return v;
 }
 
-__global__ void __launch_bounds__(128) k_gen_edge(const nzb_gen_mesh m, const nzb_physics ph, const double* __restrict__ U,
-                                                  double* __restrict__ fw, double* __restrict__ smax) {
+__global__ void __launch_bounds__(128) k_gen_edge(const nzb_gen_mesh m, const nzb_physics ph, const double* U, double* fw,
+                                                  double* smax) {
   chain_release();
   const int64_t n_edge = m.n_int + m.n_bnd;
   const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -121,14 +121,14 @@ __global__ void __launch_bounds__(128) k_gen_edge(const nzb_gen_mesh m, const nz
       for (int i = 0; i < np; ++i) {
         const double b = __ldg(bl + i * nqf);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) UL[s] = fma(b, __ldg(Ul + i * 4 + s), UL[s]);
+        for (int s = 0; s < 4; ++s) UL[s] = fma(b, Ul[i * 4 + s], UL[s]);
       }
       if (interior) {
 #pragma unroll 4
         for (int i = 0; i < np; ++i) {
           const double b = __ldg(br + i * nqf);
 #pragma unroll
-          for (int s = 0; s < 4; ++s) UR[s] = fma(b, __ldg(Ur + i * 4 + s), UR[s]);
+          for (int s = 0; s < 4; ++s) UR[s] = fma(b, Ur[i * 4 + s], UR[s]);
         }
       }
       const double nx = m.edge_normal[(k * nqf + q) * 2], ny = m.edge_normal[(k * nqf + q) * 2 + 1];

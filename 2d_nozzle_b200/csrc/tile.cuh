@@ -391,6 +391,10 @@ __device__ __forceinline__ double quad_min(double v) {
 // arrays are read before the wait, so a launch is chained only where the call itself
 // put a kernel of the chain in front of it -- never right after work of the caller's
 // (which may have written them, as nzb_geometry does).
+// Whatever a kernel of the chain writes (states, lambda, the RK4 rates, edge fluxes, local steps) is read
+// by ordinary loads after the wait: the read-only path (__ldg, or const __restrict__ on a kernel's
+// parameter) holds for data that nothing writes while the kernel is resident, and the compiler may move
+// such a load across the wait.  It is for the mesh, the tables and an adjoint's frozen state.
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -425,6 +429,11 @@ __device__ __forceinline__ void copy_rows(double* dst, const double* __restrict_
     if (r + (lane >> 3) < rows)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + r * 64), "l"(p + r * stride), "r"(bytes) : "memory");
   }
+}
+// Copy one double of this lane (zero where !ok) to dst.
+__device__ __forceinline__ void copy_one(double* dst, const double* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Wait until at most N of this thread's committed groups are in flight, then for the warp's other lanes.

@@ -17,7 +17,11 @@
 //            leave the own trace in the even and the neighbour's in the odd
 //            accumulator column of the lane that evaluates that face point; the
 //            weighted flux is the k-step of the lift.  The next slot's scattered
-//            loads are in flight while this slot's fluxes are evaluated.  Both
+//            loads are in flight while this slot's fluxes are evaluated, the
+//            neighbours' nodes on their way to shared memory (cp.async): as
+//            ordinary loads into registers they spilled (a residual of 10^6
+//            cubic triangles 541 -> 569 us, the 72-member sweep's 51 steps
+//            25.2 -> 28.2 ms).  Both
 //            elements of an edge form both traces from the same edge nodes, in
 //            the same order, with the same table, owner's trace left, owner's
 //            normal: bit-identical fluxes, so the scheme stays conservative.
@@ -414,15 +418,15 @@ __global__ void __launch_bounds__(TILE_WARPS * 32) k_tile_superbee(const nzb_mes
 }
 
 // What a lane reads for its point of a face slot: the neighbour's edge node of its
-// k-step, and the edge's normal, |dX/dsigma| and length.
+// k-step -- to its own places oth[32 s + lane] in shared memory -- and the edge's
+// normal, |dX/dsigma| and length.
 template <int K, int P>
 struct FacePoint {
   int code, nb, k;  // of the face this lane's point lies on; k < 0: no face
-  double oth[4];    // k-step operand
   double nx, ny, jac, len;
 
   // ccode, cnb, ck: the connectivity of face l of the element (one face per lane)
-  __device__ __forceinline__ void load(const nzb_mesh& m, const double* __restrict__ V, int ccode, int cnb, int ck, int fs,
+  __device__ __forceinline__ void load(const nzb_mesh& m, const double* V, double* oth, int ccode, int cnb, int ck, int fs,
                                        int lane) {
     using S = Shape<K, P>;
     constexpr unsigned long long EN = packed_edge_nodes<K, P>();
@@ -433,17 +437,14 @@ struct FacePoint {
     nb = __shfl_sync(0xffffffffu, cnb, src);
     k = __shfl_sync(0xffffffffu, ck, src);
     const int64_t E = m.n_elem, plane = S::NP * E;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) oth[s] = 0.0;
     nx = ny = jac = len = 0.0;
     if (f >= S::NF) k = -1;
-    if (k < 0) return;
-    if (j < S::NE && nb >= 0) {
-      const int nn = (int)(EN >> (16 * ((code >> 1) & 7) + 4 * j)) & 15;
-      const double* p = V + (nn * E + nb);
+    const bool other = k >= 0 && j < S::NE && nb >= 0;
+    const int nn = (int)(EN >> (16 * ((code >> 1) & 7) + 4 * j)) & 15;
+    const double* p = V + (other ? nn * E + nb : 0);
 #pragma unroll
-      for (int s = 0; s < 4; ++s) oth[s] = __ldg(p + s * plane);
-    }
+    for (int s = 0; s < 4; ++s) copy_one(oth + 32 * s + lane, p + s * plane, other);
+    if (k < 0) return;
     const double* eg = m.edge_geo + 4 * (int64_t)k;
     nx = __ldg(eg);
     ny = __ldg(eg + 1);
@@ -461,7 +462,8 @@ struct TileSmem {
   static constexpr int FRAGS = Tile<K, P>::STAGED * 32;
   static constexpr int STATE = S::NP * 4 * TILE_E;
   static constexpr int BUF = STATE + TileGeo<K, AFF>::ROWS * TILE_E;
-  static constexpr int WARP = 2 * BUF + (LIM ? STATE : 0);
+  static constexpr int OTHER = 4 * 32;  // the neighbours' nodes of one face slot
+  static constexpr int WARP = 2 * BUF + (LIM ? STATE : 0) + OTHER;
   static constexpr int BYTES = (FRAGS + TILE_WARPS * WARP) * 8;
   // resident blocks per SM: what the shared memory allows (1 KB of it reserved per block), at most
   // three (168 registers a thread)
@@ -486,6 +488,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
   const double* fr = smem + lane - first * 32;  // fragment n of this lane is fr[32 n]
   double* const wbuf = smem + L::FRAGS + warp * L::WARP;
   const double* const start = wbuf + 2 * L::BUF + (lane >> 2);  // this element's column of the starting state
+  double* const oth = wbuf + L::WARP - L::OTHER;
   const int64_t blocks = m.fwd_blocks ? m.n_fwd_blocks : (E + TILE_EB - 1) / TILE_EB;
   const bool stage = LIM && w.op == OP_STAGE;
 
@@ -548,10 +551,10 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
       } else {
         // the step's starting state is read last: its rows travel meanwhile
         const bool later = stage && w.stage > 1;
+        FacePoint<K, P> fp;
+        fp.load(m, w.V, oth, mycode, mynb, myk, 0, lane);
         if (later) copy_rows(wbuf + 2 * L::BUF, w.U0, S::NP * 4, E, e0, E);
         copy_commit();
-        FacePoint<K, P> fp;
-        fp.load(m, w.V, mycode, mynb, myk, 0, lane);
         double scale_t = 0.0;  // the local step, or what it is formed from
         if (stage && act) scale_t = later ? w.dt[e] : __ldg(m.area + e);
         double acc[T::NT][4][2];
@@ -627,7 +630,6 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
             }
           }
         }
-        if (more) fetch(b + gridDim.x, wbuf + cur * L::BUF);
 
         // ---- faces
         // triangles' rates: the face term carries -1/det (the rate is -M^-1 R with M = det M_ref)
@@ -635,6 +637,12 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
         double wave = 0.0;
 #pragma unroll 1
         for (int fs = 0; fs < T::FS; ++fs) {
+          // this slot's neighbour nodes have landed (the next tile's rows, asked for after the second slot's
+          // nodes, may still be on their way)
+          if (fs == 1 && more)
+            copy_wait<1>();
+          else
+            copy_wait<0>();
           constexpr unsigned long long EN = packed_edge_nodes<K, P>();
           double d[4][2];
 #pragma unroll
@@ -647,13 +655,17 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
 #pragma unroll
             for (int s = 0; s < 4; ++s) mma(d[s], own ? p[s * S::NP * 8] : 0.0, bo);
 #pragma unroll
-            for (int s = 0; s < 4; ++s) mma(d[s], fp.oth[s], bn);
+            for (int s = 0; s < 4; ++s) mma(d[s], oth[32 * s + lane], bn);
           }
           const int code = fp.code, nb = fp.nb;
           const bool valid = fp.k >= 0 && (P == 1 || l < S::NQF);
           const double nx = fp.nx, ny = fp.ny, jac = fp.jac, len = fp.len;
           // the next slot's scattered loads go out before this slot's fluxes
-          if (fs + 1 < T::FS) fp.load(m, w.V, mycode, mynb, myk, fs + 1, lane);
+          if (fs + 1 < T::FS) {
+            fp.load(m, w.V, oth, mycode, mynb, myk, fs + 1, lane);
+            copy_commit();
+          }
+          if (fs == 0 && more) fetch(b + gridDim.x, wbuf + cur * L::BUF);
           double F[4] = {0.0, 0.0, 0.0, 0.0}, sp = 0.0;
           if (valid) {
             const bool side = code & 1;
