@@ -143,6 +143,8 @@ class AdjointModel:
         if self._node_items is None:
             flat, item = torch.sort(self.elem_nodes_t.T.reshape(-1), stable=True)
             start = torch.searchsorted(flat, torch.arange(self._n_node + 1, device=self.device))
+            # done before anybody can pick them up: the next call may come on another stream
+            torch.cuda.current_stream(self.device).synchronize()
             self._node_items = (start, item)
         start, item = self._node_items
         out = torch.zeros((n_node, 2), dtype=torch.float64, device=self.device)

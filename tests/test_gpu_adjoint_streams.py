@@ -1,0 +1,35 @@
+"""What an AdjointModel builds at its first use and keeps is complete for callers on any stream."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def test_node_items_are_there_for_another_stream(cuda):
+    """The first coordinate product on a busy stream, the second right after it on another one."""
+    import torch
+
+    cfg, mesh = pkg("config"), pkg("mesh")
+    topo, xf, rf = mesh.channel_topology("quad", nx=64, nr=33)
+    ops = pkg("operators").build_operators(topo, mesh.rectangle_coords(xf, rf), 1)
+    m = pkg("adjoint").AdjointModel(ops, cfg.FlowConditions(), cfg.SolverOptions())
+    gv = np.random.default_rng(1).standard_normal((2, m.NV, m.E))
+    n = m.X0.shape[0]
+    ref = np.zeros((n, 2))
+    for c in range(2):
+        np.add.at(ref[:, c], m.elem_nodes.T, gv[c])
+    g = torch.as_tensor(gv, device=m.device)
+    torch.cuda.synchronize()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(20_000_000)  # some 10 ms
+        first = m._node_sums(g, n)
+    with torch.cuda.stream(other):
+        second = m._node_sums(g, n)
+    torch.cuda.synchronize()
+    assert np.array_equal(first.cpu().numpy(), ref) and np.array_equal(second.cpu().numpy(), ref)
