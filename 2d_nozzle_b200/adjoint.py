@@ -115,9 +115,16 @@ class AdjointModel:
             return (self._mesh_away(X) if far else self.mesh), value if on_device else pb
         return self._mesh_away(X), float(p_back) if on_device else pb
 
+    def _node_coords(self, X):
+        """X as device node coordinates: the kernels index them by the elements' nodes."""
+        Xd = X.detach().to(device=self.device, dtype=torch.float64).contiguous()
+        if Xd.ndim != 2 or Xd.shape[1] != 2 or Xd.shape[0] < self._n_node:
+            raise IndexError(f"node coordinates have shape {tuple(Xd.shape)}; the elements use {self._n_node} nodes")
+        return Xd
+
     def _mesh_away(self, X):
         # the metric terms at X are rebuilt on the device (nzb_geometry); the connectivity is this mesh's
-        Xd = X.detach().to(device=self.device, dtype=torch.float64)
+        Xd = self._node_coords(X)
         if self._other[0] is None or not torch.equal(self._other[0], Xd):
             mesh = self._other[1]
             if mesh is None:
@@ -129,9 +136,7 @@ class AdjointModel:
 
     def verts(self, X):
         """(2 NV, E) vertex coordinates of every element."""
-        Xd = X.detach().to(device=self.device, dtype=torch.float64).contiguous()
-        if Xd.ndim != 2 or Xd.shape[1] != 2 or Xd.shape[0] < self._n_node:
-            raise IndexError(f"node coordinates have shape {tuple(Xd.shape)}; the elements use {self._n_node} nodes")
+        Xd = self._node_coords(X)
         out = torch.empty((2 * self.NV, self.E), dtype=torch.float64, device=self.device)
         capi.check(self.lib.nzb_element_vertices(Xd.data_ptr(), self.elem_nodes_t.data_ptr(), self.E, self.NV,
                                                  out.data_ptr(), self.stream), "nzb_element_vertices")
