@@ -308,6 +308,7 @@ SIGNATURES = [
     ("nzb_batch_destroy", C.c_int, [P]),
     ("nzb_vjp", C.c_int, [C.POINTER(Mesh), C.POINTER(Physics), C.POINTER(AdjointArgs), P]),
     ("nzb_reciprocals", C.c_int, [P, P, P, I64, P]),
+    ("nzb_roots", C.c_int, [P, P, I64, P]),
     ("nzb_all_close", C.c_int, [P, P, I64, C.c_double, C.c_double, P, P]),
     ("nzb_element_vertices", C.c_int, [P, P, I64, C.c_int, P, P]),
     ("nzb_node_sums", C.c_int, [P, P, P, I64, I64, P, P]),

@@ -536,7 +536,12 @@ __global__ void __launch_bounds__(NT) k_reciprocals(const double* __restrict__ a
   const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
   if (t >= n) return;
   rcp[t] = lean_rcp(a[t]);
-  root[t] = lean_rsqrt(a[t]);
+  lean_sqrt(a[t], root[t]);
+}
+
+__global__ void __launch_bounds__(NT) k_roots(const double* __restrict__ a, double* __restrict__ root, int64_t n) {
+  const int64_t t = (int64_t)blockIdx.x * NT + threadIdx.x;
+  if (t < n) root[t] = lean_sqrt(a[t]);
 }
 
 // ---- node coordinates of the differentiable residual ---------------------------------
@@ -1221,6 +1226,12 @@ int nzb_reciprocals(const double* a, double* rcp, double* rsqrt, int64_t n, void
   if (!a || !rcp || !rsqrt || n <= 0) return fail("reciprocals: bad arguments");
   k_reciprocals<<<(unsigned)blocks_for(n), NT, 0, (cudaStream_t)stream>>>(a, rcp, rsqrt, n);
   return launch_check("reciprocals launch");
+}
+
+int nzb_roots(const double* a, double* root, int64_t n, void* stream) {
+  if (!a || !root || n <= 0) return fail("roots: bad arguments");
+  k_roots<<<(unsigned)blocks_for(n), NT, 0, (cudaStream_t)stream>>>(a, root, n);
+  return launch_check("roots launch");
 }
 
 int nzb_all_close(const double* a, const double* b, int64_t n, double rtol, double atol, double* flag, void* stream) {

@@ -3,11 +3,11 @@
 //
 // A division or square root is an iterative sequence of a dozen and more
 // instructions and over 100 cycles of latency (a 1 / x chain measured 135 cycles a
-// step, sqrt 103, against 13 for a multiply-add), and they are most of a flux.  One
-// reciprocal gives both traces' 1 / rho; the Roe weights need only
-// r = sqrt(rho_R / rho_L); a square root whose reciprocal is wanted too, or whose
-// argument is known positive, comes as x / sqrt(x).  HLLC goes from 11 divisions and
-// roots to 8, Roe from 7 (10 inside the entropy fix) to 4, AUSM+-up from 6 to 4.
+// step, sqrt 103, against 13 for a multiply-add), and they are most of a flux.  The Roe
+// weights need only r = sqrt(rho_R / rho_L), and reciprocals and roots are the short ones
+// below.  Each takes its own: one reciprocal of a product for two denominators (both
+// traces' 1 / rho, the star state's) has as many multiply-adds, three roundings where one
+// is enough, and overflows where neither denominator does.
 // Together with shorter address arithmetic in the loads, a residual of 480 000 linear
 // triangles went 199 -> 173 us, of 240 000 cubic quadrilaterals 235 -> 195 us (tile
 // kernel before its asynchronous copies).  The values differ from the templates' in the last
@@ -19,28 +19,44 @@
 
 namespace nzb {
 
-// 1 / a and 1 / sqrt(a) for normal, finite a (a > 0 for the root): the hardware's
-// approximation (rcp / rsqrt.approx.ftz.f64, about 20 bits) and one third-order
-// Householder step -- with e = 1 - a x,  x (1 + e + e^2), and with e = 1 - a y^2,
-// y (1 + e / 2 + 3 e^2 / 8) -- whose remainder, of order e^3 = 2^-60, is below the
-// rounding.  No range checks and no branch, unlike the division and root they
-// replace: three and four multiply-adds (nzb_reciprocals exposes them to the tests).
-// Over 4 x 10^6 arguments per decade, 1e-30 to 1e30, the reciprocal is at most one
-// unit in the last place from the division's, the root's relative error at most
-// 1.26 x 2^-53.  A stage of 480 000 cubic triangles went 380 -> 332 us with them, of
-// 240 000 cubic quadrilaterals 291 -> 260, the 72-member sweep's step 547 -> 493.  An argument of zero, a denormal or an infinity gives a NaN; the floors
-// and guards of the callers keep them above 1e-20, and a NaN stays one.
+// 1 / a, sqrt(a) and 1 / sqrt(a) for normal, finite a (a > 0 for the roots) from the hardware's
+// approximations x, y (rcp / rsqrt.approx.ftz.f64, about 20 bits).  The reciprocal takes one third-order
+// Householder step: with e = 1 - a x,  x (1 + e + e^2), whose remainder e^3 = 2^-60 is below the rounding.
+// The root is s = a y and two Heron steps s + (a - s^2) y / 2, which square the relative error and then
+// multiply it by y's: 2^-59; both residuals come exact from a multiply-add, so one rounding is left, as
+// in the division and root they replace, without their range checks and branch.  The root's reciprocal is
+// a Householder step on 1 - s y.
+// Over 4 x 10^6 arguments per decade, 1e-30 to 1e30, reciprocal and root are the division's and sqrt's
+// but for one unit in the last place at 4 of 10^4 (nzb_reciprocals and nzb_roots expose them to the tests).
+// With the first such forms a stage of 480 000 cubic triangles went 380 -> 332 us, of 240 000 cubic
+// quadrilaterals 291 -> 260, the 72-member sweep's step 547 -> 493; these, with a rounding fewer a root and
+// two fewer a pair of denominators, take 1 % more of the sweep (51 steps 25.1 -> 25.4 ms).
+// Arguments of zero, a denormal or an infinity give a NaN; the floors and guards of the callers keep them
+// above 1e-10, and a NaN stays one.
 __device__ __forceinline__ double lean_rcp(double a) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
   const double e = fma(-a, x, 1.0);
   return fma(x, fma(e, e, e), x);
 }
-__device__ __forceinline__ double lean_rsqrt(double a) {
+__device__ __forceinline__ double rsqrt_approx(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-(a * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
+  return y;
+}
+__device__ __forceinline__ double root_from(double a, double y) {
+  const double h = 0.5 * y;
+  double s = a * y;
+  s = fma(fma(-s, s, a), h, s);
+  return fma(fma(-s, s, a), h, s);
+}
+__device__ __forceinline__ double lean_sqrt(double a) { return root_from(a, rsqrt_approx(a)); }
+// sqrt(a), and its reciprocal in rcp
+__device__ __forceinline__ double lean_sqrt(double a, double& rcp) {
+  const double y = rsqrt_approx(a), s = root_from(a, y);
+  const double e = fma(-s, y, 1.0);
+  rcp = fma(y, fma(e, e, e), y);
+  return s;
 }
 
 // primitives(U, g) of physics.cuh with lean_rcp.
@@ -55,45 +71,21 @@ __device__ __forceinline__ Prim lean_primitives(const double* U, double g) {
   return s;
 }
 
-struct PrimPair {
-  Prim L, R;
-};
-
-__device__ __forceinline__ PrimPair primitive_pair(const double* UL, const double* UR, double g) {
-  PrimPair s;
-  s.L.rho = floor_at(UL[0], FLOOR);
-  s.R.rho = floor_at(UR[0], FLOOR);
-  const double t = lean_rcp(s.L.rho * s.R.rho);
-  s.L.inv = t * s.R.rho;
-  s.R.inv = t * s.L.rho;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    Prim& q = k ? s.R : s.L;
-    const double* U = k ? UR : UL;
-    q.vx = U[1] * q.inv;
-    q.vy = U[2] * q.inv;
-    q.p = floor_at((g - 1.0) * (U[3] - 0.5 * q.rho * (q.vx * q.vx + q.vy * q.vy)), FLOOR);
-    q.H = (U[3] + q.p) * q.inv;
-  }
-  return s;
-}
-
 __device__ __forceinline__ double lean_roe_flux(const double* UL, const double* UR, double nx, double ny, double g,
                                            double efix, double* F) {
-  const PrimPair s = primitive_pair(UL, UR, g);
-  const Prim &L = s.L, &R = s.R;
+  const Prim L = lean_primitives(UL, g), R = lean_primitives(UR, g);
   double FL[4], FR[4];
   normal_flux(L, nx, ny, FL);
   normal_flux(R, nx, ny, FR);
-  const double r2 = R.rho * L.inv;
-  const double r = r2 * lean_rsqrt(r2);
+  const double r = lean_sqrt(R.rho * L.inv);
   const double iden = lean_rcp(1.0 + r);
   const double vx = (L.vx + r * R.vx) * iden;
   const double vy = (L.vy + r * R.vy) * iden;
   const double H = (L.H + r * R.H) * iden;
   const double q2 = vx * vx + vy * vy;
   const double c2 = floor_at((g - 1.0) * (H - 0.5 * q2), FLOOR);
-  const double ic = lean_rsqrt(c2), c = c2 * ic;
+  double ic;
+  const double c = lean_sqrt(c2, ic);
   const double vn = vx * nx + vy * ny;
   double l1 = fabs(vn + c), l2 = fabs(vn - c), l3 = fabs(vn);
   const double smax = l1 < l2 ? l2 : l1;
@@ -119,21 +111,17 @@ __device__ __forceinline__ double lean_roe_flux(const double* UL, const double* 
 
 __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double* UR, double nx, double ny, double g,
                                             double low_mach, double* F) {
-  const PrimPair s = primitive_pair(UL, UR, g);
-  const Prim &L = s.L, &R = s.R;
+  const Prim L = lean_primitives(UL, g), R = lean_primitives(UR, g);
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
-  const double aL2 = floor_at(g * L.p * L.inv, FLOOR), aR2 = floor_at(g * R.p * R.inv, FLOOR);
-  const double aL = aL2 * lean_rsqrt(aL2), aR = aR2 * lean_rsqrt(aR2);
-  const double r2 = R.rho * L.inv;
-  const double r = r2 * lean_rsqrt(r2);
+  const double aL = lean_sqrt(floor_at(g * L.p * L.inv, FLOOR)), aR = lean_sqrt(floor_at(g * R.p * R.inv, FLOOR));
+  const double r = lean_sqrt(R.rho * L.inv);
   const double iden = lean_rcp(1.0 + r);
   const double vx = (L.vx + r * R.vx) * iden;
   const double vy = (L.vy + r * R.vy) * iden;
   const double H = (L.H + r * R.H) * iden;
   const double vt = vx * nx + vy * ny;
-  const double at2 = floor_at((g - 1.0) * (H - 0.5 * (vx * vx + vy * vy)), FLOOR);
-  const double at = at2 * lean_rsqrt(at2);
+  const double at = lean_sqrt(floor_at((g - 1.0) * (H - 0.5 * (vx * vx + vy * vy)), FLOOR));
   double SL = fmin(vnL - aL, vt - at);
   double SR = fmax(vnR + aR, vt + at);
   if (low_mach > 0.0) {
@@ -159,12 +147,9 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
   F[2] = mf * uy + p * ny;
   F[3] = vn * (E + p);
   if (star) {
-    // U* - U with one reciprocal for 1 / (S - SM) and 1 / (rho (S - vn))
-    const double a = guard(S - SM), b = guard(m);
-    const double t = lean_rcp(a * b);
-    const double rs = m * (t * b);  // rho (S - vn) / (S - SM)
+    const double rs = m * lean_rcp(guard(S - SM));  // rho (S - vn) / (S - SM)
     const double dv = SM - vn;
-    const double Es = E * (left ? L.inv : R.inv) + dv * (SM + p * (t * a));
+    const double Es = E * (left ? L.inv : R.inv) + dv * (SM + p * lean_rcp(guard(m)));
     F[0] += S * (rs - (left ? UL[0] : UR[0]));
     F[1] += S * (rs * (ux + dv * nx) - (left ? UL[1] : UR[1]));
     F[2] += S * (rs * (uy + dv * ny) - (left ? UL[2] : UR[2]));
@@ -176,22 +161,19 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
 __device__ __forceinline__ double lean_ausm_up_flux(const double* UL, const double* UR, double nx, double ny, double g,
                                                double* F) {
   constexpr double BETA = 0.125, ALPHA = 0.1875, KP = 0.4, KU = 0.2;
-  const PrimPair s = primitive_pair(UL, UR, g);
-  const Prim &L = s.L, &R = s.R;
+  const Prim L = lean_primitives(UL, g), R = lean_primitives(UR, g);
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
-  const double aL2 = g * L.p * L.inv, aR2 = g * R.p * R.inv;
-  const double aL = aL2 * lean_rsqrt(aL2), aR = aR2 * lean_rsqrt(aR2);
+  const double aL = lean_sqrt(g * L.p * L.inv), aR = lean_sqrt(g * R.p * R.inv);
   const double ah = 0.5 * (aL + aR), rh = 0.5 * (L.rho + R.rho);
-  const double t = lean_rcp(ah * rh), iah = t * rh;
-  const double mL = vnL * iah, mR = vnR * iah;
+  const double iah = lean_rcp(ah), mL = vnL * iah, mR = vnR * iah;
   const double mb2 = 0.5 * (mL * mL + mR * mR);
   const double pL2 = 0.25 * ((mL + 1.0) * (mL + 1.0)), mL2 = -0.25 * ((mL - 1.0) * (mL - 1.0));
   const double pR2 = 0.25 * ((mR + 1.0) * (mR + 1.0)), mR2 = -0.25 * ((mR - 1.0) * (mR - 1.0));
   const double m4p = fabs(mL) >= 1.0 ? 0.5 * (mL + fabs(mL)) : pL2 * (1.0 - 16.0 * BETA * mL2);
   const double m4m = fabs(mR) >= 1.0 ? 0.5 * (mR - fabs(mR)) : mR2 * (1.0 + 16.0 * BETA * pR2);
   const double dif = 1.0 - mb2;
-  const double uh = ah * (m4p + m4m) + KP * (dif < 0.0 ? 0.0 : dif) * (L.p - R.p) * t;
+  const double uh = ah * (m4p + m4m) + KP * (dif < 0.0 ? 0.0 : dif) * (L.p - R.p) * lean_rcp(rh * ah);
   const double p5p = fabs(mL) >= 1.0 ? (mL > 0.0 ? 1.0 : 0.0) : pL2 * ((2.0 - mL) - 16.0 * ALPHA * mL * mL2);
   const double p5m = fabs(mR) >= 1.0 ? (mR > 0.0 ? 0.0 : 1.0) : mR2 * ((-2.0 - mR) + 16.0 * ALPHA * mR * pR2);
   const double ph = p5p * L.p + p5m * R.p + KU * p5p * p5m * rh * ah * (vnL - vnR);

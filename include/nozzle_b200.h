@@ -366,6 +366,8 @@ int nzb_vjp_coords(const nzb_mesh* mesh, const nzb_physics* phys, const double* 
 /* 1 / a and 1 / sqrt(a) of positive normal numbers as the kernels' fluxes form them (csrc/flux.cuh), for
  * checking their accuracy. */
 int nzb_reciprocals(const double* a, double* rcp, double* rsqrt, int64_t n, void* stream);
+/* ... and sqrt(a) of positive normal numbers. */
+int nzb_roots(const double* a, double* root, int64_t n, void* stream);
 /* Helpers of the differentiable residual's coordinate product.  nzb_all_close sets *flag = 1 where some
  * |a - b| > atol + rtol |b| (the caller zeroes it).  nzb_element_vertices writes the (2 NV, E) vertex
  * coordinates nzb_vjp_coords takes from (n_node, 2) coordinates and (E, NV) vertex ids (all in range).
