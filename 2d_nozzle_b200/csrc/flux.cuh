@@ -58,6 +58,12 @@ __device__ __forceinline__ double lean_sqrt(double a, double& rcp) {
   rcp = fma(y, fma(e, e, e), y);
   return s;
 }
+// A sound speed from its square s = lean_sqrt(a): an infinite one (infinite energy) stays infinite, so the
+// local step it bounds is zero.
+__device__ __forceinline__ double sound_speed(double a, double s) {
+  return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000 ? a : s;
+}
+__device__ __forceinline__ double sound_speed(double a) { return sound_speed(a, lean_sqrt(a)); }
 
 // primitives(U, g) of physics.cuh with lean_rcp.
 __device__ __forceinline__ Prim lean_primitives(const double* U, double g) {
@@ -85,7 +91,7 @@ __device__ __forceinline__ double lean_roe_flux(const double* UL, const double* 
   const double q2 = vx * vx + vy * vy;
   const double c2 = floor_at((g - 1.0) * (H - 0.5 * q2), FLOOR);
   double ic;
-  const double c = lean_sqrt(c2, ic);
+  const double c = sound_speed(c2, lean_sqrt(c2, ic));
   const double vn = vx * nx + vy * ny;
   double l1 = fabs(vn + c), l2 = fabs(vn - c), l3 = fabs(vn);
   const double smax = l1 < l2 ? l2 : l1;
@@ -114,7 +120,7 @@ __device__ __forceinline__ double lean_hllc_flux(const double* UL, const double*
   const Prim L = lean_primitives(UL, g), R = lean_primitives(UR, g);
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
-  const double aL = lean_sqrt(floor_at(g * L.p * L.inv, FLOOR)), aR = lean_sqrt(floor_at(g * R.p * R.inv, FLOOR));
+  const double aL = sound_speed(floor_at(g * L.p * L.inv, FLOOR)), aR = sound_speed(floor_at(g * R.p * R.inv, FLOOR));
   const double r = lean_sqrt(R.rho * L.inv);
   const double iden = lean_rcp(1.0 + r);
   const double vx = (L.vx + r * R.vx) * iden;
@@ -164,7 +170,7 @@ __device__ __forceinline__ double lean_ausm_up_flux(const double* UL, const doub
   const Prim L = lean_primitives(UL, g), R = lean_primitives(UR, g);
   const double vnL = L.vx * nx + L.vy * ny;
   const double vnR = R.vx * nx + R.vy * ny;
-  const double aL = lean_sqrt(g * L.p * L.inv), aR = lean_sqrt(g * R.p * R.inv);
+  const double aL = sound_speed(g * L.p * L.inv), aR = sound_speed(g * R.p * R.inv);
   const double ah = 0.5 * (aL + aR), rh = 0.5 * (L.rho + R.rho);
   const double iah = lean_rcp(ah), mL = vnL * iah, mR = vnR * iah;
   const double mb2 = 0.5 * (mL * mL + mR * mR);

@@ -644,9 +644,11 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
           else
             copy_wait<0>();
           constexpr unsigned long long EN = packed_edge_nodes<K, P>();
-          double d[4][2];
+          // the own trace in column 0, the neighbour's in column 1 of an accumulator of its own: in one they
+          // would meet the other's zero columns, and an infinity times zero is a NaN
+          double d[4][2], dn[4][2];
 #pragma unroll
-          for (int s = 0; s < 4; ++s) d[s][0] = d[s][1] = 0.0;
+          for (int s = 0; s < 4; ++s) d[s][0] = d[s][1] = dn[s][0] = dn[s][1] = 0.0;
           {
             const int f = P == 1 ? 2 * fs + (l >> 1) : fs, j = P == 1 ? (l & 1) : l;
             const bool own = f < S::NF && j < S::NE;
@@ -655,7 +657,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
 #pragma unroll
             for (int s = 0; s < 4; ++s) mma(d[s], own ? p[s * S::NP * 8] : 0.0, bo);
 #pragma unroll
-            for (int s = 0; s < 4; ++s) mma(d[s], oth[32 * s + lane], bn);
+            for (int s = 0; s < 4; ++s) mma(dn[s], oth[32 * s + lane], bn);
           }
           const int code = fp.code, nb = fp.nb;
           const bool valid = fp.k >= 0 && (P == 1 || l < S::NQF);
@@ -673,8 +675,8 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, (TileSmem<K, P, AFF, LIM>::MI
               double L4[4], R4[4];
 #pragma unroll
               for (int s = 0; s < 4; ++s) {
-                L4[s] = side ? d[s][1] : d[s][0];
-                R4[s] = side ? d[s][0] : d[s][1];
+                L4[s] = side ? dn[s][1] : d[s][0];
+                R4[s] = side ? d[s][0] : dn[s][1];
               }
               sp = lean_interface_flux(L4, R4, nx, ny, ph, F);
             } else {
