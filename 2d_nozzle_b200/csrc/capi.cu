@@ -47,6 +47,25 @@ static bool tables_ready(int kind, int order) {
   return g_tab_done.count({dev, kind * 16 + order}) != 0;
 }
 
+// The tile kernels take a quadrilateral's Jacobian from its bilinear coefficients (TileGeo), so they need
+// the unit square's vertex functions in the uploaded tables; with others, split = 4 runs the one-thread
+// kernels, which read the functions' derivatives from the tables.
+static std::set<std::pair<int, int>> g_tile_off;  // (device, kind * 16 + order) whose tables are not the unit square's
+
+static bool unit_square(int order, const double* slot) {
+  return order == 1 ? unit_square_tables<1>(slot) : order == 2 ? unit_square_tables<2>(slot) : unit_square_tables<3>(slot);
+}
+static bool tile_kernels(int kind, int order) {
+  if (order < 1) return false;
+  if (kind == NZB_TRI) return true;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_tab_mu);
+  return g_tile_off.count({dev, kind * 16 + order}) == 0;
+}
+static bool tile_forward(const nzb_mesh& m) { return m.split == TILE_LANES && tile_kernels(m.kind, m.order); }
+static bool tile_adjoint(const nzb_mesh& m) { return m.vjp_split == TILE_LANES && tile_kernels(m.kind, m.order); }
+
 static int check_mesh(const nzb_mesh* m) {
   if (!m) return fail("mesh is null");
   if (m->kind != NZB_TRI && m->kind != NZB_QUAD) return fail("unknown element kind");
@@ -81,11 +100,11 @@ static int block_threads(int kind, int order) {
 // Elements per block of the forward element kernel: 32 with four lanes per
 // element, else one per thread.
 static int element_width(const nzb_mesh& m) {
-  return (m.split == TILE_LANES && m.order > 0) ? TILE_EB : block_threads(m.kind, m.order);
+  return tile_forward(m) ? TILE_EB : block_threads(m.kind, m.order);
 }
 // ... and of the adjoint state kernel.
 static int adjoint_width(const nzb_mesh& m) {
-  return (m.vjp_split == TILE_LANES && m.order > 0) ? TILE_EB : block_threads(m.kind, m.order);
+  return tile_adjoint(m) ? TILE_EB : block_threads(m.kind, m.order);
 }
 // Blocks of the forward element kernel (= norm partial slots of stage 1).
 static int64_t element_blocks(const nzb_mesh& m) { return (m.n_elem + element_width(m) - 1) / element_width(m); }
@@ -117,7 +136,15 @@ static int dispatch(const nzb_mesh& m, const nzb_physics& ph, const Work& w, cud
     if (!m.elem_share || !m.lim_means || !m.lim_scale)
       return fail("the Superbee limiter needs elem_share, lim_means and lim_scale");
   }
-  const cudaError_t e = m.kind == NZB_TRI ? element_launch_tri(m, ph, w, st) : element_launch_quad(m, ph, w, st);
+  nzb_mesh one;
+  const nzb_mesh* run = &m;
+  if (m.split == TILE_LANES && m.order > 0 && !tile_forward(m)) {
+    one = m;
+    one.split = 1;
+    one.edge_pass = 0;  // split = 4 ignores it
+    run = &one;
+  }
+  const cudaError_t e = m.kind == NZB_TRI ? element_launch_tri(*run, ph, w, st) : element_launch_quad(*run, ph, w, st);
   return cuda_check(e, "element kernel launch");
 }
 
@@ -481,7 +508,14 @@ static int batch_graph(Batch& B, int n, int first, cudaGraphExec_t* out) {
 static int dispatch_vjp(const nzb_mesh& m, const nzb_physics& ph, const AdjWork& w, cudaStream_t st) {
   if (adjoint_blocks(m) > 0x7fffffff) return fail("too many elements for one launch");
   if (check_block_list(m.vjp_blocks, m.n_vjp_blocks, adjoint_blocks(m), w.norm_partial, "vjp_blocks")) return -1;
-  const cudaError_t e = m.kind == NZB_TRI ? vjp_launch_tri(m, ph, w, st) : vjp_launch_quad(m, ph, w, st);
+  nzb_mesh one;
+  const nzb_mesh* run = &m;
+  if (m.vjp_split == TILE_LANES && !tile_adjoint(m)) {
+    one = m;
+    one.vjp_split = 1;
+    run = &one;
+  }
+  const cudaError_t e = m.kind == NZB_TRI ? vjp_launch_tri(*run, ph, w, st) : vjp_launch_quad(*run, ph, w, st);
   return cuda_check(e, "vjp kernel launch");
 }
 
@@ -751,19 +785,24 @@ int nzb_upload_tables(int kind, int order, const double* tables, int64_t n) {
   if (!tables) return fail("tables is null");
   // every translation unit holds its own copy of the tables
   const size_t off = (size_t)slot_offset(kind, order);
+  const bool tiles = order > 0 && (kind == NZB_TRI || unit_square(order, tables));
   if (cuda_check(cudaMemcpyToSymbol(c_tab, tables, sizeof(double) * n, sizeof(double) * off), "table upload") ||
       cuda_check(upload_tables_fwd_tri(tables, (size_t)n, off), "table upload (triangles)") ||
       cuda_check(upload_tables_fwd_quad(tables, (size_t)n, off), "table upload (quadrilaterals)") ||
       cuda_check(upload_tables_tri(tables, (size_t)n, off), "table upload (adjoint, triangles)") ||
       cuda_check(upload_tables_quad(tables, (size_t)n, off), "table upload (adjoint, quadrilaterals)") ||
-      cuda_check(kind == NZB_TRI ? upload_tiles_fwd_tri(order, tables) : upload_tiles_fwd_quad(order, tables),
-                 "tile fragment upload") ||
-      cuda_check(kind == NZB_TRI ? upload_tiles_vjp_tri(order, tables) : upload_tiles_vjp_quad(order, tables),
-                 "adjoint tile fragment upload"))
+      (tiles && (cuda_check(kind == NZB_TRI ? upload_tiles_fwd_tri(order, tables) : upload_tiles_fwd_quad(order, tables),
+                            "tile fragment upload") ||
+                 cuda_check(kind == NZB_TRI ? upload_tiles_vjp_tri(order, tables) : upload_tiles_vjp_quad(order, tables),
+                            "adjoint tile fragment upload"))))
     return -1;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(g_tab_mu);
+  if (tiles || order == 0)
+    g_tile_off.erase({dev, kind * 16 + order});
+  else
+    g_tile_off.insert({dev, kind * 16 + order});
   g_tab_done.insert({dev, kind * 16 + order});
   return 0;
 }
@@ -1321,7 +1360,7 @@ int nzb_adjoint_create(int n_buckets, const nzb_mesh* meshes, const nzb_physics*
 }
 
 int64_t nzb_adjoint_jacobian_doubles(const nzb_mesh* mesh) {
-  if (!mesh || mesh->vjp_split != TILE_LANES || mesh->order < 1 || mesh->n_elem < 1) return 0;
+  if (!mesh || !tile_adjoint(*mesh) || mesh->n_elem < 1) return 0;
   return mesh->kind == NZB_TRI ? vjp_jac_doubles_tri(mesh->order, mesh->n_elem)
                                : vjp_jac_doubles_quad(mesh->order, mesh->n_elem);
 }

@@ -62,7 +62,7 @@ struct Tile {
 
   // Fragment numbers (32 doubles each).  The point -> node tables come plain (residuals), before the
   // common part, and folded with the constant factor of the inverse mass (rates, stages), after it, so
-  // what a kernel stages in shared memory is one range: [0, COMMON_END) or [COMMON, COUNT).
+  // what a kernel stages in shared memory is one range: [0, COMMON_END) or [COMMON, COMMON + COMMON_END).
   static constexpr int VXN = VS * NT * 2, LFN = FS * NT;  // fragments of one VX / LF table
   static constexpr int COMMON = VXN + LFN;
   static constexpr int PHI = COMMON;                // [VT][NS] nodes -> volume points
@@ -285,7 +285,7 @@ std::vector<double> tile_tables(const double* slot) {
 }
 
 // Whether a quadrilateral slot's vertex shape derivatives are those of the unit
-// square with vertices (0,0), (1,0), (0,1), (1,1), as the kernels assume.
+// square with vertices (0,0), (1,0), (0,1), (1,1), as the tile kernels assume.
 template <int P>
 bool unit_square_tables(const double* slot) {
   using S = Shape<1, P>;
@@ -314,9 +314,6 @@ __device__ __forceinline__ void stage_tiles(double* dst, int first, int n) {
 // Build and upload the fragments of one (kind, order) from its table slot into this unit's copy.
 template <int K, int P>
 static cudaError_t upload_tiles(const double* slot) {
-  if constexpr (K == 1) {
-    if (!unit_square_tables<P>(slot)) return cudaErrorInvalidValue;
-  }
   const std::vector<double> t = tile_tables<K, P>(slot);
   const size_t off = sizeof(double) * (size_t)tile_offset<K>(P);
   return K == 0 ? cudaMemcpyToSymbol(g_tile_tri, t.data(), sizeof(double) * t.size(), off)

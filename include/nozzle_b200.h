@@ -168,7 +168,9 @@ typedef struct {
 
 /* Tables of one reference element: see the packer in layout.py for the order.
  * Must be called once per device and (kind, order) before any other call on
- * that kind and order.  Host pointer. */
+ * that kind and order.  Host pointer.  Quadrilateral tables whose vertex
+ * functions are not the unit square's run on the one-thread kernels (split = 4
+ * and vjp_split = 4 then mean 1). */
 int nzb_upload_tables(int kind, int order, const double* tables, int64_t n);
 /* Number of doubles nzb_upload_tables expects for (kind, order). */
 int64_t nzb_table_size(int kind, int order);
