@@ -22,7 +22,8 @@ both above p = 0: a stage of a single solve takes 7-14 us with it and 25-220 us
 with one thread per element, a step of a 72-member sweep (211 680 elements) 0.49
 against 1.0 ms.  Within a context the variant is fixed per (kind, order), never
 per mesh; a batch built with ``variants="single"`` runs the plain solve's kernels
-and gives its bits.  One exception, :func:`bucket_context`.
+and gives its bits.  One exception, with a table of its own (``lone``): a batch's large
+instance on an arbitrary state (:func:`arbitrary_state`).
 
 The table is ``variants.json`` beside this module, written by
 ``python -m 2d_nozzle_b200.autotune --write`` on a B200 (see :func:`tune`).
@@ -55,7 +56,7 @@ DEFAULT = {("tri", 0): "t1", ("tri", 1): "t1_edge", ("tri", 2): "split4", ("tri"
 
 CONTEXTS = ("single", "batch")
 # table keys per context: forward and adjoint variants
-_KEYS = {("single", "fwd"): "choice", ("batch", "fwd"): "batch_choice",
+_KEYS = {("single", "fwd"): "choice", ("batch", "fwd"): "batch_choice", ("lone", "fwd"): "lone_choice",
          ("single", "vjp"): "vjp_choice", ("batch", "vjp"): "batch_vjp_choice"}
 
 
@@ -67,8 +68,9 @@ def table_path() -> str:
 
 def load_table(path: str | None = None, context: str = "single", which: str = "fwd") -> dict:
     """(kind, order) -> variant name for a context, from the measured table (or the defaults).  A table
-    without the batch entries uses its single-solve ones for batches too."""
-    if context not in CONTEXTS:
+    without the batch entries uses its single-solve ones for batches too, one without the ``lone`` entries
+    its batch ones there."""
+    if (context, which) not in _KEYS:
         raise ValueError(f"context {context!r}: use one of {CONTEXTS}")
     path = path or table_path()
     names = VARIANTS if which == "fwd" else VJP_VARIANTS
@@ -76,7 +78,11 @@ def load_table(path: str | None = None, context: str = "single", which: str = "f
     if os.path.exists(path):
         with open(path) as fh:
             data = json.load(fh)
-        entries = data.get(_KEYS[(context, which)]) or data.get(_KEYS[("single", which)], {})
+        entries = data.get(_KEYS[(context, which)])
+        if not entries and context == "lone":
+            entries = data.get(_KEYS[("batch", which)])
+        if not entries:
+            entries = data.get(_KEYS[("single", which)], {})
         for key, name in entries.items():
             kind, order = key.split(":")
             if name not in names:
@@ -103,8 +109,6 @@ def variant_for(kind: str, order: int, context: str = "single") -> str:
         if forced not in VARIANTS:
             raise ValueError(f"NZB_VARIANT={forced!r}: use one of {sorted(VARIANTS)}")
         return forced
-    if context == "lone":
-        return "t1"
     name = _lookup(kind, order, context, "fwd")
     # four lanes per element apply from p = 1 up
     return "t1" if (name == "split4" and int(order) == 0) else name
@@ -162,17 +166,28 @@ def context_for(n_elem: int, variants: str = "auto") -> str:
     return variants
 
 
-# Elements above which the only instance of a bucket keeps the one-thread kernels (bucket_context).
+# Elements above which an arbitrary state in a batch keeps the one-thread kernels (arbitrary_state).
 LONE_ELEMENTS = 16384
 
 
+def arbitrary_state(inst) -> bool:
+    """Whether a batch's instance is a large mesh on a state that no nozzle came with (no ``geometry``): it
+    gets a bucket of its own and the ``lone`` table, the one-thread kernels, whoever marches beside it and
+    to its last step.  Such states can be ill-conditioned without bound: of random ones the limiter
+    rescales half the elements toward vacuum (to 1e-8 of the average), which leaves their density and
+    pressure eight digits fewer and the speeds formed from them likewise.  Over 64 of them, 20 000 to
+    500 000 elements, one limited step of the tile kernel and one of the one-thread kernel differ by 4e-13
+    in the median, by 1.6e-8 in one of ten and by 4.7e-6 at most (against a plain 64-bit evaluation either
+    was 1e-11 to 2e-10 off on three states, and the one-thread kernel 2.4e-4 on a fourth); the design
+    sweep's states by 9e-15.  Results on such states therefore stay bit for bit, although the tile kernel
+    is faster there (500 000 cubic triangles: a limited stage 1.03 against 0.55 ms).  Below the line a mesh
+    does not fill the GPU and the tile kernel's shorter path is worth more (a stage of 4 480 cubic
+    quadrilaterals 44 against 14 us)."""
+    return inst.geometry is None and int(inst.ops.n_elem) > LONE_ELEMENTS
+
+
 def bucket_context(n_instances: int, n_elem: int, variants: str) -> str:
-    """The variant context of a batch's bucket: ``variants``, except that a throughput bucket holding a
-    single large instance takes ``lone``, whose forward choice is the one-thread kernel.  One large mesh
-    of random states, half of whose elements the limiter rescales toward vacuum, magnifies the last bits
-    of the fluxes by up to 1e8 in one step (a contact speed equal to a wave speed but for round-off), so
-    such a batch keeps its results bit for bit although the tile kernel is faster there (500 000 cubic
-    triangles: a limited stage 1.03 against 0.55 ms).  Sweeps' instances are far below the line (9 000 elements at refinement 3)."""
+    """The variant context of a bucket of arbitrary states (:func:`arbitrary_state`; one instance each)."""
     return "lone" if variants == "batch" and n_instances == 1 and n_elem > LONE_ELEMENTS else variants
 
 
@@ -457,6 +472,7 @@ def tune(device="cuda:0", reps: int = 5, grad_elements: int = 143_360) -> dict:
     for k in KINDS:
         for c in ("choice", "batch_choice"):
             doc[c][f"{k}:0"] = "t1"
+    doc["lone_choice"] = {f"{k}:{o}": "t1" for k in KINDS for o in ORDERS}  # not a matter of time: arbitrary_state
     return doc
 
 

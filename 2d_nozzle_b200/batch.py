@@ -28,7 +28,7 @@ import numpy as np
 
 from . import capi
 from .config import FLUX_IDS, SCHEMES, recommended_scheme, residual_scale, step_coefficient
-from .autotune import bucket_context, choose_variant, set_struct_variant, tail_elements
+from .autotune import arbitrary_state, bucket_context, choose_variant, set_struct_variant, tail_elements
 from .layout import DeviceMesh, concat_arrays, host_arrays, physics_struct
 
 STATUS = {0: "running", 1: "converged", 2: "non-finite", 3: "diverged", 4: "stalled", 5: "max_iterations"}
@@ -91,9 +91,10 @@ class BatchSolver:
         self.device = dev
         n = len(instances)
 
-        # buckets of one (kind, order)
-        keys = [(inst.ops.ref.kind, inst.ops.ref.order) for inst in instances]
-        self.bucket_keys = sorted(set(keys), key=lambda k: (k[0], k[1]))
+        # buckets of one (kind, order); a large arbitrary state has one to itself (third entry: its index)
+        keys = [(inst.ops.ref.kind, inst.ops.ref.order, i if variants == "batch" and arbitrary_state(inst) else -1)
+                for i, inst in enumerate(instances)]
+        self.bucket_keys = sorted(set(keys))
         self.members = [[i for i in range(n) if keys[i] == k] for k in self.bucket_keys]
         begin = np.zeros(n, np.int64)
         end = np.zeros(n, np.int64)
@@ -186,7 +187,7 @@ class BatchSolver:
                 dm.pack(U0, S[0])
                 self.h2d_bytes += U0.nbytes
             self.U0_soa.append(S[0].clone())
-            choose_variant(dm, bucket_context(len(mem), dm.E, variants))
+            choose_variant(dm, variants if key[2] < 0 else bucket_context(len(mem), dm.E, variants))
             self.h2d_bytes += sum(a.nbytes for a in arrays.values() if isinstance(a, np.ndarray))
             bf = capi.Buffers()
             bf.S0, bf.S1, bf.S2 = (x.data_ptr() for x in S)
@@ -266,10 +267,10 @@ class BatchSolver:
         and, with ``running`` (a per-instance mask), each bucket's list of the blocks that hold elements
         of running instances (None without)."""
         meshes, lists = [], []
-        for dm, mem in zip(self.meshes, self.members):
+        for key, dm, mem in zip(self.bucket_keys, self.meshes, self.members):
             mc = capi.Mesh()
             C.memmove(C.byref(mc), C.byref(dm.c), C.sizeof(capi.Mesh))
-            if context is not None:
+            if context is not None and key[2] < 0:  # an arbitrary state's kernels stay
                 set_struct_variant(mc, dm.kind, dm.order, context)
             blocks = None
             if running is not None:
