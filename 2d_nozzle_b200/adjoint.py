@@ -35,7 +35,7 @@ from . import capi
 from . import nozzle as nz
 from .backend import B200Backend
 from .config import SolverOptions, step_coefficient
-from .autotune import choose_variant, context_for, set_struct_variant, tail_elements
+from .autotune import choose_variant, context_for, same_kernels, set_struct_variant, tail_elements
 from .layout import DeviceMesh, face_tangent_table, physics_struct
 from .march import solve as march_solve
 from .mesh import INFLOW, OUTFLOW
@@ -702,8 +702,8 @@ class BatchGradient:
         either way: its seed, step and march depend on its own converged state
         only.  In the default batch context the forward and adjoint marches
         switch to the single-solve variants for their tails (few elements still
-        marching), at a point that depends on the whole batch, so the two
-        orders agree to round-off.
+        marching) where the table has other ones there, at a point that depends
+        on the whole batch, so the two orders agree to round-off.
         """
         from .batch import BatchSolver, blocks_of
 
@@ -797,11 +797,13 @@ class BatchGradient:
             return hh.value, int(blocks.size)
 
         # Late in the march (few members left, or few blocks holding them) the adjoint switches to the
-        # single-solve variant and to a march object that lists only the blocks of members still
-        # marching or yet to start, as the forward batch does (BatchSolver._retarget).
+        # single-solve variant, where that is another one, and to a march object that lists only the
+        # blocks of members still marching or yet to start, as the forward batch does
+        # (BatchSolver._retarget).
         first_h, launched = adjoint_handle(None, None)
         cur = [first_h]
-        tail_at = tail_elements() if self.variants == "batch" else 0
+        switches = not same_kernels(mesh, dm.kind, dm.order, "single", "vjp")
+        tail_at = tail_elements() if self.variants == "batch" and switches else 0
         in_tail = False
         self.tail_switched = {"forward": None, "adjoint": None}
         self.compactions = {"forward": 0, "adjoint": 0}

@@ -147,6 +147,15 @@ def set_struct_variant(mc, kind: str, order: int, context: str) -> None:
     mc.vjp_split = VJP_VARIANTS[vjp_variant_for(kind, order, context)] if order > 0 else 1
 
 
+def same_kernels(mc, kind: str, order: int, context: str, which: str) -> bool:
+    """Whether a mesh struct's forward (``fwd``) or adjoint (``vjp``) kernels are already those of a context."""
+    other = capi.Mesh()
+    set_struct_variant(other, kind, order, context)
+    if which == "vjp":
+        return mc.vjp_split == other.vjp_split
+    return (mc.split, bool(mc.edge_pass)) == (other.split, bool(other.edge_pass))
+
+
 def tail_elements() -> int:
     """Active elements below which a batch switches to the single-solve variants: with fewer, one thread
     (or four) per active element no longer fills a B200 (148 SMs x 8 resident warps of 32 threads at the

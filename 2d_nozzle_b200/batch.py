@@ -28,7 +28,7 @@ import numpy as np
 
 from . import capi
 from .config import FLUX_IDS, SCHEMES, recommended_scheme, residual_scale, step_coefficient
-from .autotune import arbitrary_state, bucket_context, choose_variant, set_struct_variant, tail_elements
+from .autotune import arbitrary_state, bucket_context, choose_variant, same_kernels, set_struct_variant, tail_elements
 from .layout import DeviceMesh, concat_arrays, host_arrays, physics_struct
 
 STATUS = {0: "running", 1: "converged", 2: "non-finite", 3: "diverged", 4: "stalled", 5: "max_iterations"}
@@ -246,11 +246,13 @@ class BatchSolver:
         # Late in a march most instances have retired.  Two things follow, both taken between chunks when
         # the set of running instances has changed: (1) once the instances still marching hold few
         # elements, the batch's throughput variants leave the GPU idle and an element's latency decides,
-        # so the march switches to the single-solve variants (the tail); (2) once the blocks holding
+        # so the march switches to the single-solve variants (the tail), where these are other ones; (2) once the blocks holding
         # running elements are at most half of those a launch spans, a march object whose launches list
         # only those blocks replaces the current one, so a launch no longer walks every retired block.
         self.variants = variants
-        self._tail_at = tail_elements() if variants == "batch" else 0
+        switches = [key[2] < 0 and not same_kernels(dm.c, dm.kind, dm.order, "single", "fwd")
+                    for key, dm in zip(self.bucket_keys, self.meshes)]
+        self._tail_at = tail_elements() if variants == "batch" and any(switches) else 0
         self.compact = bool(compact)
         self._in_tail = False
         self._launched = self._blocks_launched(None, None)
