@@ -324,15 +324,17 @@ class AdjointMarch:
                                                      offs.ctypes.data, C.byref(am), C.byref(h)), "nzb_adjoint_create")
         self.am = am
         self.handle = h.value
-        self.jac = _jacobian_workspace(self.model.lib, self.model.mesh.c, self.model.device)
-        capi.check(self.model.lib.nzb_adjoint_jacobians(h, 0, self.jac.data_ptr() if self.jac is not None else None),
-                   "nzb_adjoint_jacobians")
 
     def __del__(self):
         if getattr(self, "handle", None):
             self.model.lib.nzb_adjoint_destroy(self.handle)
 
     def run(self, n_steps: int) -> tuple[int, float, float, int]:
+        if n_steps > 0 and not hasattr(self, "jac"):  # the defect alone needs no workspace
+            self.jac = _jacobian_workspace(self.model.lib, self.model.mesh.c, self.model.device)
+            capi.check(self.model.lib.nzb_adjoint_jacobians(self.handle, 0,
+                                                            self.jac.data_ptr() if self.jac is not None else None),
+                       "nzb_adjoint_jacobians")
         capi.check(self.model.lib.nzb_adjoint_run(self.handle, int(n_steps), self.model.stream), "nzb_adjoint_run")
         return (int(self.t["status"].item()), float(self.t["res"].item()), float(self.t["res0"].item()),
                 int(self.t["iterations"].item()))
