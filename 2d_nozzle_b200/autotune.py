@@ -50,8 +50,7 @@ KINDS = ("tri", "quad")
 TABLE_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "variants.json")
 
 # used when variants.json is absent
-DEFAULT = {("tri", 0): "t1", ("tri", 1): "t1_edge", ("tri", 2): "split4", ("tri", 3): "split4",
-           ("quad", 0): "t1", ("quad", 1): "t1_edge", ("quad", 2): "split4", ("quad", 3): "split4"}
+DEFAULT = {(k, p): "split4" if p else "t1" for k in KINDS for p in ORDERS}
 
 
 CONTEXTS = ("single", "batch")
@@ -124,7 +123,7 @@ def apply_variant(mesh, name: str) -> None:
 # chosen per (kind, order) and context from the same table; NZB_VJP_VARIANT
 # forces one.
 VJP_VARIANTS = {"t1": 1, "split4": 4}
-VJP_DEFAULT = {(k, p): "t1" for k in KINDS for p in ORDERS}
+VJP_DEFAULT = dict(DEFAULT)
 
 
 def vjp_variant_for(kind: str, order: int, context: str = "single") -> str:
@@ -209,39 +208,54 @@ def choose_variant(mesh, context: str = "single") -> str:
     return name
 
 
-def measure_vjp(mesh, phys, state, reps: int = 5) -> dict:
-    """Microseconds of one adjoint RK4 stage (the march's unit of work: the transposed product, the rate
-    and the stage update) on ``mesh`` for each adjoint variant (best of ``reps``); the mesh's own variant
-    is restored afterwards."""
+def measure_vjp(mesh, phys, state, reps: int = 5, steps: int = 25) -> dict:
+    """Microseconds of one RK4 stage of an adjoint march (the transposed product, the rate and the stage
+    update) on ``mesh`` for each adjoint variant, as a run of ``steps`` steps takes it: with the face
+    Jacobians formed at the run's start where the variant stores them, and the check at its end (best of
+    ``reps``).  The mesh's own variant is restored afterwards."""
+    import numpy as np
     import torch
 
     lib = capi.load()
-    n = state.numel()
-    lam, seed, out, f0, f1, f2 = (torch.zeros(n, dtype=torch.float64, device=mesh.device) for _ in range(6))
-    seed.normal_(generator=torch.Generator(device=mesh.device).manual_seed(0))
-    dt = torch.full((mesh.E,), 1e-3, dtype=torch.float64, device=mesh.device)
-    a = capi.AdjointArgs()
-    a.mode, a.stage = capi.ADJ_RK4, 1
-    a.U, a.lam, a.seed, a.out = state.data_ptr(), seed.data_ptr(), seed.data_ptr(), out.data_ptr()
-    a.lam0, a.dt, a.f0, a.f1, a.f2 = lam.data_ptr(), dt.data_ptr(), f0.data_ptr(), f1.data_ptr(), f2.data_ptr()
-    stream = torch.cuda.current_stream(mesh.device)
+    dev, n = mesh.device, state.numel()
+    z = lambda n, t=torch.float64: torch.zeros(n, dtype=t, device=dev)  # noqa: E731
+    lam, seed, Y1, Y2, f0, f1, f2 = (z(n) for _ in range(7))
+    seed.normal_(generator=torch.Generator(device=dev).manual_seed(0))
+    dt = torch.full((mesh.E,), 1e-6, dtype=torch.float64, device=dev)
+    bf = capi.AdjointBuffers()
+    for name, t in (("U", state), ("seed", seed), ("lam", lam), ("Y1", Y1), ("Y2", Y2), ("f0", f0), ("f1", f1),
+                    ("f2", f2), ("dt", dt)):
+        setattr(bf, name, t.data_ptr())
+    record = {"inst_begin": z(1, torch.int64), "inst_end": torch.full((1,), mesh.E, dtype=torch.int64, device=dev),
+              "inst_count": torch.ones(1, dtype=torch.float64, device=dev), "elem_norm": z(mesh.E),
+              "status": z(1, torch.int32), "iterations": z(1, torch.int32), "res0": z(1), "res": z(1),
+              "n_running": z(1, torch.int32)}
+    am = capi.AdjointMarch()
+    am.n_inst, am.tolerance, am.max_iterations = 1, 0.0, 2**31 - 1
+    for name, t in record.items():
+        setattr(am, name, t.data_ptr())
+    offs = np.zeros(1, np.int64)
+    stream = torch.cuda.current_stream(dev)
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
     keep = mesh.vjp_split
     res = {}
     for name, threads in VJP_VARIANTS.items():
         mesh.vjp_split = threads
-
-        def run():
-            capi.check(lib.nzb_vjp(C.byref(mesh.c), C.byref(phys), C.byref(a), stream.cuda_stream), "nzb_vjp")
-
-        run()
-        t = []
-        for _ in range(reps):
-            ev[0].record(stream)
-            run()
-            ev[1].record(stream)
-            ev[1].synchronize()
-            t.append(1e3 * ev[0].elapsed_time(ev[1]))
+        h = capi.P()
+        capi.check(lib.nzb_adjoint_create(1, C.byref(mesh.c), C.byref(phys), C.byref(bf), offs.ctypes.data, C.byref(am),
+                                          C.byref(h)), "nzb_adjoint_create")
+        try:
+            t = []
+            for k in range(reps + 1):
+                lam.zero_()
+                ev[0].record(stream)
+                capi.check(lib.nzb_adjoint_run(h, steps, stream.cuda_stream), "nzb_adjoint_run")
+                ev[1].record(stream)
+                ev[1].synchronize()
+                if k:  # the first run captures its graph
+                    t.append(1e3 * ev[0].elapsed_time(ev[1]) / (4 * steps))
+        finally:
+            lib.nzb_adjoint_destroy(h)
         res[name] = {"rk4_stage_us": min(t)}
     mesh.vjp_split = keep
     return res
@@ -402,13 +416,13 @@ def _batch_step_seconds(insts, table: dict, device, chunks: int = 3) -> float:
 def tune(device="cuda:0", reps: int = 5, grad_elements: int = 143_360) -> dict:
     """Measure the variants per (kind, order) in both contexts; returns the table document.
 
-    * single solve (``choice``, ``vjp_choice``): one SSP-RK3 first and second stage and one adjoint RK4
-      stage of every variant on one design-sweep instance per mesh size, each on its own mesh (a plain
+    * single solve (``choice``, ``vjp_choice``): one SSP-RK3 first and second stage and an adjoint march's
+      RK4 stage of every variant on one design-sweep instance per mesh size, each on its own mesh (a plain
       solve's latency);
     * batch (``batch_choice``): coordinate descent over the buckets' forward variants, each candidate
       timed as whole steps of the sampled 256-point sweep's batch (every bucket marching side by side:
       throughput); a change is kept when it saves more than 1 %;
-    * batch adjoint (``batch_vjp_choice``): the adjoint RK4 stage on the sweep's bucket of that element
+    * batch adjoint (``batch_vjp_choice``): an adjoint march's RK4 stage on the sweep's bucket of that element
       type and on a unit rectangle of ``grad_elements`` elements (the batched gradients' bucket size).
     """
     import torch
