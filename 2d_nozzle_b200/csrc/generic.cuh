@@ -26,8 +26,8 @@
 //                  screen, probe values held in shared memory, 12-step pressure
 //                  bisection).
 //
-// What bounds a stage: the operators are the element's own (7.8 KB for a
-// fourth-order triangle, 34 KB at p = 5), so they are read once, each by one warp, as
+// What bounds a stage: the operators are the element's own (7.8 KB read for a
+// fourth-order triangle, 15 KB at p = 5), so they are read once, each by one warp, as
 // FP64 mma A fragments: rows are nodes, a k-step four consecutive points of a
 // row (32 contiguous bytes a row), the B operand the four components of the point
 // fluxes (half its columns are unused, which costs nothing where loads decide).
